@@ -386,8 +386,8 @@ int level_begin(pm_handle* h, const LevelBufs& B, const uint8_t* left, const uin
     PM_CUDA(h, cudaMemsetAsync(B.Rs, 0, N * 16, st));
     launch_view_clear(B.vb1c, B.vb1s, N, st);
     launch_view_clear(B.vb2c, B.vb2s, N, st);
-    launch_pack_tex(B.texL, B.Lbw, B.Lg, W, H, st);
-    launch_pack_tex(B.texR, B.Rbw, B.Rg, W, H, st);
+    launch_pack_tex(B.texL, B.Lbw, B.Lg, W, H, F, st);
+    launch_pack_tex(B.texR, B.Rbw, B.Rg, W, H, F, st);
     prof_mark(h, st, PM_PHASE_PREP, 6);
     // init (:469-470, :349-379): a given disparity without normals gets normals from it
     int nl = 0;
@@ -513,8 +513,8 @@ int run_depth(pm_handle* h, void* ws, const uint8_t* left, const uint8_t* right,
     launch_view_clear(vb2c, vb2s, N, st);   // :212
     float4* texL = at<float4>(ws, L, Layout::texL);
     float4* texR = at<float4>(ws, L, Layout::texR);
-    launch_pack_tex(texL, Lc, Lg, W, H, st);
-    launch_pack_tex(texR, Rc, Rg, W, H, st);
+    launch_pack_tex(texL, Lc, Lg, W, H, F, st);
+    launch_pack_tex(texR, Rc, Rg, W, H, F, st);
     prof_mark(h, st, PM_PHASE_PREP, 6);
     int nl = 0;
     const float4* initn = initnormal;
@@ -798,13 +798,14 @@ struct TexPair {
     float4* t1 = nullptr;
     float4* t2 = nullptr;
     cudaStream_t st = nullptr;
-    int make(const float* bw1, const float* g1, const float* bw2, const float* g2, int W, int H, cudaStream_t s)
+    int make(const float* bw1, const float* g1, const float* bw2, const float* g2, int W, int H, int fused,
+             cudaStream_t s)
     {
         st = s;
         PM_CUDA(nullptr, cudaMallocAsync((void**)&t1, tex_bytes(W, H), s));
         PM_CUDA(nullptr, cudaMallocAsync((void**)&t2, tex_bytes(W, H), s));
-        launch_pack_tex(t1, (const float4*)bw1, (const float4*)g1, W, H, s);
-        launch_pack_tex(t2, (const float4*)bw2, (const float4*)g2, W, H, s);
+        launch_pack_tex(t1, (const float4*)bw1, (const float4*)g1, W, H, fused, s);
+        launch_pack_tex(t2, (const float4*)bw2, (const float4*)g2, W, H, fused, s);
         return PM_OK;
     }
     ViewData view(int W, int H, int r) const { return make_view(t1, t2, W, H, r); }
@@ -1660,7 +1661,7 @@ int pm_k_init(float* out, const float* bw1, const float* bw2, const float* g1, c
     if (rc) return rc;
     if (!out || !bw1 || !bw2 || !g1 || !g2 || (initdisp && !initnormal)) return fail(nullptr, PM_EINVAL_ARG, "null argument");
     TexPair tp;
-    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, S(stream)))) return rc;
+    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, fused, S(stream)))) return rc;
     const ViewData V = tp.view(W, H, r);
     launch_init((float4*)out, V, dmax, lr, initdisp, (const float4*)initnormal, fused, S(stream));
     PM_CUDA(nullptr, cudaGetLastError());
@@ -1674,7 +1675,7 @@ int pm_k_cost(float* cost, const float* planes, const float* bw1, const float* b
     if (rc) return rc;
     if (!cost || !planes || !bw1 || !bw2 || !g1 || !g2) return fail(nullptr, PM_EINVAL_ARG, "null argument");
     TexPair tp;
-    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, S(stream)))) return rc;
+    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, fused, S(stream)))) return rc;
     const ViewData V = tp.view(W, H, r);
     launch_cost(cost, (const float4*)planes, V, mincost, fused, S(stream));
     PM_CUDA(nullptr, cudaGetLastError());
@@ -1688,7 +1689,7 @@ int pm_k_klt(float* out, const float* planes, const float* bw1, const float* bw2
     if (rc) return rc;
     if (!out || !planes || !bw1 || !bw2 || !g1 || !g2) return fail(nullptr, PM_EINVAL_ARG, "null argument");
     TexPair tp;
-    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, S(stream)))) return rc;
+    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, fused, S(stream)))) return rc;
     const ViewData V = tp.view(W, H, r);
     launch_klt((float4*)out, (const float4*)planes, V, fused, S(stream));
     PM_CUDA(nullptr, cudaGetLastError());
@@ -1709,7 +1710,7 @@ int pm_k_propagate(float* out, const float* old, const float* bw1, const float* 
     if (!d_err) PM_CUDA(nullptr, cudaMalloc(&d_err, sizeof(int)));
     PropParams P;
     TexPair tp;
-    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, S(stream)))) return rc;
+    if ((rc = tp.make(bw1, g1, bw2, g2, W, H, fused, S(stream)))) return rc;
     P.V = tp.view(W, H, r);
     P.out = (float4*)out;
     P.old = (const float4*)old;

@@ -197,8 +197,9 @@ __device__ __forceinline__ float expf_neg(float x)
     p = fmaf(p, r, 0.5f);
     p = fmaf(p, r, 1.0f);
     p = fmaf(p, r, 1.0f);
-    const int ni = __float_as_int(t) - __float_as_int(M);   // n as an integer, in [-126, 0]
-    return p * __int_as_float((ni + 127) << 23);
+    // p 2^n by adding n to p's exponent field: the bits of t are those of M plus n, and the bits of M
+    // vanish in the shift
+    return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
 }
 
 // support weight exp(-|dot(I1(q) - I1(p), gray)| * 12) (:355, :701, :1491).  Colours are

@@ -82,11 +82,11 @@ __global__ void k_prep(const uint8_t* __restrict__ img, size_t stride, int W, in
     }
 }
 
-template <bool F, bool CHK>
+template <bool F, bool GEN>
 __global__ void k_init(float4* __restrict__ out, ViewData V, float dmax, int lr, const float* __restrict__ initdisp,
                        const float4* __restrict__ initnormal, int dual)
 {
-    if (variant_skips<CHK>(V, dual)) return;
+    if (variant_skips<GEN>(V, dual)) return;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= V.W || y >= V.H) return;
     const size_t i = (size_t)y * V.W + x;
@@ -105,31 +105,31 @@ __global__ void k_init(float4* __restrict__ out, ViewData V, float dmax, int lr,
         ret = nd_state_init(rng, cx, cy, lr, dmax);
     }
     Counters cnt = {0, 0, 0, 0};
-    ret.w = patch_eval<F, false, CHK>(V, x, y, ret, 1e10f, cnt);
+    ret.w = patch_eval<F, false, GEN>(V, x, y, ret, 1e10f, cnt);
     out[i] = ret;
 }
 
-template <bool F, bool CHK>
+template <bool F, bool GEN>
 __global__ void k_cost(float* __restrict__ cost, const float4* __restrict__ planes, ViewData V, float mincost,
                        int dual)
 {
-    if (variant_skips<CHK>(V, dual)) return;
+    if (variant_skips<GEN>(V, dual)) return;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= V.W || y >= V.H) return;
     const size_t i = (size_t)y * V.W + x;
     Counters cnt = {0, 0, 0, 0};
-    cost[i] = patch_eval<F, false, CHK>(V, x, y, planes[i], mincost, cnt);
+    cost[i] = patch_eval<F, false, GEN>(V, x, y, planes[i], mincost, cnt);
 }
 
-template <bool F, bool CHK>
+template <bool F, bool GEN>
 __global__ void k_klt(float4* __restrict__ out, const float4* __restrict__ planes, ViewData V, int dual)
 {
-    if (variant_skips<CHK>(V, dual)) return;
+    if (variant_skips<GEN>(V, dual)) return;
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= V.W || y >= V.H) return;
     const size_t i = (size_t)y * V.W + x;
     Counters cnt = {0, 0, 0, 0};
-    out[i] = klt2<F, false, CHK>(V, x, y, planes[i], cnt);
+    out[i] = klt2<F, false, GEN>(V, x, y, planes[i], cnt);
 }
 
 __device__ __forceinline__ void normal_depth_px(float4* __restrict__ out, const float4* __restrict__ planes, int W,
@@ -669,26 +669,68 @@ __global__ void k_disparity_to_normal(float4* __restrict__ out, const float* __r
     out[(size_t)y * W + x] = f4(n.x, n.y, n.z, 0.0f);
 }
 
-// texel planes of one view (pm_window.cuh): column c in [-2, W+1] of the colour plane
-// holds bw, of the gradient plane grad, of the compact plane (bw.rgb, gradient sign
-// a finite nonzero colour value below 2^-40 in magnitude (the window loops then need the
-// exact-division fallback of ad_sum)
-__device__ __forceinline__ bool tiny_colour(float v) { return v != 0.0f && fabsf(v) < 0x1p-40f; }
+// whether a colour value is byte / 255, and that byte
+__device__ __forceinline__ bool unorm_byte(float v, uint32_t& k)
+{
+    const float x = v * 255.0f;
+    k = x >= 0.0f && x <= 255.0f ? (uint32_t)__float2int_rn(x) : 0u;
+    return __float_as_uint((float)k / 255.0f) == __float_as_uint(v);
+}
 
-// bytes), all of column clamp(c, 0, W-1)
+// The pair plane's sign threshold of one gradient component (PairRec): the smallest A in
+// [0, 2^15) for which the component interpolated at a = A 2^-15 has another sign than texel
+// i's, PAIR_NEVER if there is none.  Exact for weights between the grid points too: equal
+// signs interpolate to that sign for every a < 1; for opposite signs the two rounded products
+// grow and shrink monotonically in a, so the sign of their sum changes once.
+template <bool F>
+__device__ __forceinline__ uint32_t pair_threshold(float g0, float g1)
+{
+    const uint32_t s0 = __float_as_uint(g0) >> 31;
+    if (s0 == __float_as_uint(g1) >> 31) return PAIR_NEVER;
+    uint32_t lo = 0, hi = PAIR_NEVER;   // the answer lies in [lo, hi]
+#pragma unroll 1
+    while (lo < hi) {
+        const uint32_t m = (lo + hi) >> 1;
+        const float a = (float)m * 0x1p-15f, b = 1.0f - a;
+        const float v = F ? fmaf(a, g1, b * g0) : b * g0 + a * g1;
+        if (__float_as_uint(v) >> 31 != s0) hi = m;
+        else lo = m + 1;
+    }
+    return lo;
+}
+
+// texel planes of one view (pm_window.cuh): column c in [-4, W+3] of the colour plane holds bw,
+// of the gradient plane grad, of the compact plane (bw.rgb, gradient sign bytes), all of
+// column clamp(c, 0, W-1), and of the pair plane the record of columns clamp(c), clamp(c + 1)
+template <bool F>
 __global__ void k_pack_tex(float4* __restrict__ tex, const float4* __restrict__ bw, const float4* __restrict__ grad,
                            int W, int H, int P)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x - TEX_PAD, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (c > W + TEX_PAD - 1 || y >= H) return;
-    const int s = min(max(c, 0), W - 1);
-    const size_t o = (size_t)y * P + c + TEX_PAD;
+    const int s = min(max(c, 0), W - 1), s1 = min(max(c + 1, 0), W - 1);
+    const size_t o = (size_t)y * P + c + TEX_PAD, plane = (size_t)H * P;
     const float4 col = bw[(size_t)y * W + s], g = grad[(size_t)y * W + s];
+    const float4 col1 = bw[(size_t)y * W + s1], g1 = grad[(size_t)y * W + s1];
+    const uint32_t sb = sign_bytes(g);
     tex[o] = col;
-    tex[(size_t)H * P + o] = g;
-    tex[(size_t)2 * H * P + o] = make_float4(col.x, col.y, col.z, __uint_as_float(sign_bytes(g)));
-    if (c == s && (tiny_colour(col.x) || tiny_colour(col.y) || tiny_colour(col.z)))
-        atomicOr(reinterpret_cast<int*>(tex + (size_t)3 * H * P), 1);
+    tex[plane + o] = g;
+    tex[2 * plane + o] = make_float4(col.x, col.y, col.z, __uint_as_float(sb));
+    uint32_t k[6];
+    bool ok = unorm_byte(col.x, k[0]);
+    ok &= unorm_byte(col.y, k[1]);
+    ok &= unorm_byte(col.z, k[2]);
+    unorm_byte(col1.x, k[3]);
+    unorm_byte(col1.y, k[4]);
+    unorm_byte(col1.z, k[5]);
+    ok &= fin(g.x) && fin(g.y) && fin(g.z) && fin(g.w);
+    PairRec R;
+    R.x = k[0] | k[1] << 8 | k[2] << 16 | signbits4(g) << 24;
+    R.y = k[3] | k[4] << 8 | k[5] << 16;
+    R.z = pair_threshold<F>(g.y, g1.y) | pair_threshold<F>(g.w, g1.w) << 16;
+    R.w = pair_threshold<F>(g.x, g1.x) | pair_threshold<F>(g.z, g1.z) << 16;
+    reinterpret_cast<PairRec*>(tex)[3 * plane + o] = R;
+    if (c == s && !ok) atomicOr(reinterpret_cast<int*>(tex + TEX_PLANES * plane), 1);
 }
 
 __global__ void k_view_clear(int* __restrict__ count, unsigned long long* __restrict__ src, size_t n)
@@ -946,13 +988,15 @@ void launch_crop(float* dst, int Wd, int Hd, const float* src, int Ws, int chann
 }
 
 int tex_pitch(int W) { return W + 2 * TEX_PAD; }
-size_t tex_bytes(int W, int H) { return ((size_t)tex_pitch(W) * H * 3 + 1) * sizeof(float4); }
+size_t tex_bytes(int W, int H) { return ((size_t)tex_pitch(W) * H * TEX_PLANES + 1) * sizeof(float4); }
 
-void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, cudaStream_t st)
+void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, int fused, cudaStream_t st)
 {
     const dim3 b(64, 4);
-    cudaMemsetAsync(tex + (size_t)3 * tex_pitch(W) * H, 0, sizeof(float4), st);   // the tiny-colour flag
-    k_pack_tex<<<grid2d(tex_pitch(W), H, b), b, 0, st>>>(tex, bw, grad, W, H, tex_pitch(W));
+    const dim3 g = grid2d(tex_pitch(W), H, b);
+    cudaMemsetAsync(tex + (size_t)TEX_PLANES * tex_pitch(W) * H, 0, sizeof(float4), st);   // the general-loop flag
+    if (fused) k_pack_tex<true><<<g, b, 0, st>>>(tex, bw, grad, W, H, tex_pitch(W));
+    else k_pack_tex<false><<<g, b, 0, st>>>(tex, bw, grad, W, H, tex_pitch(W));
 }
 
 void launch_view_clear(int* count, unsigned long long* src, size_t n, cudaStream_t st)

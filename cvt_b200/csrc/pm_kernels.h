@@ -65,7 +65,7 @@ void prop_tile_shape(int* w, int* h);
 // false for any other width
 bool prop_batch_tile_shape(int tile_w, int* w, int* h);
 // pairs per batched propagate launch: their arguments are one kernel parameter block
-// (128 x 184 bytes, within the 32,764 bytes a launch may pass)
+// (128 x 192 bytes, within the 32,764 bytes a launch may pass)
 constexpr int PROP_GROUP = 128;
 struct PropGroup {
     PropParams p[PROP_GROUP];
@@ -141,16 +141,17 @@ void launch_crop(float* dst, int Wd, int Hd, const float* src, int Ws, int chann
 // the size_t width by the float scale 0.35f and truncates
 inline int pyr_next(int n) { return (int)(size_t)((float)(size_t)n * 0.35f); }
 void launch_view_clear(int* count, unsigned long long* src, size_t n, cudaStream_t st);
-// texel planes of a view (pm_window.cuh) from its bw and grad fields
+// texel planes of a view (pm_window.cuh) from its bw and grad fields; the pair plane's sign
+// thresholds are those of the fused or of the strict interpolation
 int tex_pitch(int W);
 size_t tex_bytes(int W, int H);
 inline ViewData make_view(const float4* t1, const float4* t2, int W, int H, int r)
 {
     const int plane = tex_pitch(W) * H;
-    return ViewData{t1, t2, W, H, r, tex_pitch(W), plane, reinterpret_cast<const int*>(t1 + (size_t)3 * plane),
-                    reinterpret_cast<const int*>(t2 + (size_t)3 * plane)};
+    return ViewData{t1, t2, W, H, r, tex_pitch(W), plane, reinterpret_cast<const int*>(t1 + (size_t)TEX_PLANES * plane),
+                    reinterpret_cast<const int*>(t2 + (size_t)TEX_PLANES * plane), make_float2(1.0f, 1.0f)};
 }
-void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, cudaStream_t st);
+void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, int fused, cudaStream_t st);
 // FP32 peak probe: `iters` rounds of independent fma chains per thread
 void launch_fma_peak(float* out, int iters, int blocks, int threads, cudaStream_t st);
 double fma_peak_flops_per_iter();

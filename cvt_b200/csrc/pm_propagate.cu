@@ -28,20 +28,23 @@ namespace {
 #define PM_PROP_BY 4
 #endif
 constexpr int PROP_BX = PM_PROP_BX, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
-// resident threads per SM asked of the register allocator for each kernel (768 threads =
-// 80 registers, 640 = 96; measured best at 768 for both)
+// Resident threads per SM asked of the register allocator for each kernel: 512 = 128 registers, which
+// the pair loops (two samples in flight per thread) use without spills.  Measured at 1280x720, r = 10, 3
+// iterations, ms (chain / Gauss-Newton): 512 threads 70.2 / 97.8, 640 (96 registers, 24-40 bytes
+// spilled) 70.6 / 100.8, 768 (80 registers, 64-190 bytes) 69.6 / 106.2; at 320x240 2.50 / 3.91, 2.81 /
+// 4.57, 2.82 / 4.91: the FMA pipe is busy at 16 warps already, and short grids gain from ILP.
+// The block shape does not matter (32x4 184.7 ms a call, 16x8 185.5, 8x16 187.4, 32x2 185.9).
 #ifndef PM_CHAIN_THREADS
-#define PM_CHAIN_THREADS 768
+#define PM_CHAIN_THREADS 512
 #endif
 #ifndef PM_KLT_THREADS
-#define PM_KLT_THREADS 768
+#define PM_KLT_THREADS 512
 #endif
 constexpr int PM_CHAIN_BLOCKS = PM_CHAIN_THREADS / PROP_THREADS, PM_KLT_BLOCKS = PM_KLT_THREADS / PROP_THREADS;
-// the batched (persistent) forms read each pair's arguments from global memory instead of the
-// parameter bank, which takes registers: at 768 threads per SM they spill in the window loops,
-// so they are compiled for 640 (96 registers)
+// the batched (persistent) forms index each pair's arguments in a parameter block, which takes
+// registers; they are compiled for the same 128
 #ifndef PM_BATCH_THREADS
-#define PM_BATCH_THREADS 640
+#define PM_BATCH_THREADS 512
 #endif
 constexpr int PM_BATCH_BLOCKS = PM_BATCH_THREADS / PROP_THREADS;
 
@@ -93,7 +96,7 @@ __device__ __forceinline__ bool known_outcome(float4 nb, float4 self, float thet
 // [-4, 5] (:982-991), 6 a random plane (:996-1002), 7-8 cross-view planes (:1007-1016),
 // 9 the randomized refinement (:1021-1028).  One loop, so that the window evaluation has a
 // single call site.
-template <bool F, bool COUNT, bool CHK, int BX = PROP_BX, int BY = PROP_BY>
+template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
 __device__ __forceinline__ void chain_tile(const PropParams& P, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
@@ -145,14 +148,14 @@ __device__ __forceinline__ void chain_tile(const PropParams& P, int bx, int by, 
                 nb = nd_state_refine(rng, self, cx, cy, dmax, lr);
             }
             if (k == 0) {
-                self.w = patch_eval<F, COUNT, CHK>(V, px, py, nb, 1e10f, cnt);
+                self.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, 1e10f, cnt);
                 sd_self = smooth_dist1(self, smooth, cx, cy, dmax, lr);
             } else {
                 if (known_outcome(nb, self, theta, sd_self)) continue;
                 const float sd = smooth_dist1(nb, smooth, cx, cy, dmax, lr);
                 // minimalCost (:873-877)
                 const float mincost = self.w + theta * sd_self - theta * sd;
-                nb.w = patch_eval<F, COUNT, CHK>(V, px, py, nb, mincost, cnt);
+                nb.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, mincost, cnt);
                 if (nb.w + theta * sd <= self.w + theta * sd_self) {   // :976 etc.
                     self = nb;
                     sd_self = sd;
@@ -163,17 +166,17 @@ __device__ __forceinline__ void chain_tile(const PropParams& P, int bx, int by, 
     }
 }
 
-template <bool F, bool COUNT, bool CHK>
+template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS, PM_CHAIN_BLOCKS) k_prop_chain(PropParams P)
 {
-    if (variant_skips<CHK>(P.V, P.dual)) return;
+    if (variant_skips<GEN>(P.V, P.dual)) return;
     Counters cnt = {0, 0, 0, 0};
-    chain_tile<F, COUNT, CHK>(P, blockIdx.x, blockIdx.y, cnt);
+    chain_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
 // Gauss-Newton plane steps (:1034-1038)
-template <bool F, bool COUNT, bool CHK, int BX = PROP_BX, int BY = PROP_BY>
+template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
 __device__ __forceinline__ void klt_tile(const PropParams& P, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
@@ -181,22 +184,22 @@ __device__ __forceinline__ void klt_tile(const PropParams& P, int bx, int by, Co
     if (px < V.W && py < V.H) {
         const size_t idx = (size_t)py * V.W + px;
         float4 nb = P.tmp_self[idx];
-        for (int k = 0; k < 6; k++) nb = klt2<F, COUNT, CHK>(V, px, py, nb, cnt);
+        for (int k = 0; k < 6; k++) nb = klt2<F, COUNT, GEN>(V, px, py, nb, cnt);
         P.tmp_nb[idx] = nb;
     }
 }
 
-template <bool F, bool COUNT, bool CHK>
+template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt(PropParams P)
 {
-    if (variant_skips<CHK>(P.V, P.dual)) return;
+    if (variant_skips<GEN>(P.V, P.dual)) return;
     Counters cnt = {0, 0, 0, 0};
-    klt_tile<F, COUNT, CHK>(P, blockIdx.x, blockIdx.y, cnt);
+    klt_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
 // evaluation of the Gauss-Newton result (:1039-1052), view scatter (:1060-1067), output (:1070)
-template <bool F, bool COUNT, bool CHK, int BX = PROP_BX, int BY = PROP_BY>
+template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
 __device__ __forceinline__ void final_tile(const PropParams& P, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
@@ -214,7 +217,7 @@ __device__ __forceinline__ void final_tile(const PropParams& P, int bx, int by, 
         const float2 sd = smooth_distance(nb, self, smooth, cx, cy, dmax, lr);
         if (!known_outcome(nb, self, theta, sd.y)) {
             const float mincost = self.w + theta * sd.y - theta * sd.x;
-            nb.w = patch_eval<F, COUNT, CHK>(V, px, py, nb, mincost, cnt);
+            nb.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, mincost, cnt);
             if (nb.w + theta * sd.x <= self.w + theta * sd.y) self = nb;
         }
 
@@ -233,12 +236,12 @@ __device__ __forceinline__ void final_tile(const PropParams& P, int bx, int by, 
     }
 }
 
-template <bool F, bool COUNT, bool CHK>
+template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS) k_prop_final(PropParams P)
 {
-    if (variant_skips<CHK>(P.V, P.dual)) return;
+    if (variant_skips<GEN>(P.V, P.dual)) return;
     Counters cnt = {0, 0, 0, 0};
-    final_tile<F, COUNT, CHK>(P, blockIdx.x, blockIdx.y, cnt);
+    final_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(PROP_THREADS) k_prop_final(PropParams P)
 // parameter block (read through the constant cache, as a single-pair launch reads its own),
 // job.x indexing it.  Every pixel runs the same operations on the same fields as in a
 // single-pair launch, so the results are the same bit for bit.
-template <bool F, bool COUNT, bool CHK, int BX>
+template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_chain_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
@@ -257,14 +260,14 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
         if (j >= njobs) return;
         const uint2 job = jobs[j];
         const PropParams& P = G.p[job.x];
-        if (variant_skips<CHK>(P.V, P.dual)) continue;
+        if (variant_skips<GEN>(P.V, P.dual)) continue;
         Counters cnt = {0, 0, 0, 0};
-        chain_tile<F, COUNT, CHK, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
+        chain_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
         flush_counters<COUNT>(cnt, P.counters);
     }
 }
 
-template <bool F, bool COUNT, bool CHK, int BX>
+template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_klt_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
@@ -273,14 +276,14 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
         if (j >= njobs) return;
         const uint2 job = jobs[j];
         const PropParams& P = G.p[job.x];
-        if (variant_skips<CHK>(P.V, P.dual)) continue;
+        if (variant_skips<GEN>(P.V, P.dual)) continue;
         Counters cnt = {0, 0, 0, 0};
-        klt_tile<F, COUNT, CHK, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
+        klt_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
         flush_counters<COUNT>(cnt, P.counters);
     }
 }
 
-template <bool F, bool COUNT, bool CHK, int BX>
+template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_final_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
@@ -289,9 +292,9 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
         if (j >= njobs) return;
         const uint2 job = jobs[j];
         const PropParams& P = G.p[job.x];
-        if (variant_skips<CHK>(P.V, P.dual)) continue;
+        if (variant_skips<GEN>(P.V, P.dual)) continue;
         Counters cnt = {0, 0, 0, 0};
-        final_tile<F, COUNT, CHK, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
+        final_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
         flush_counters<COUNT>(cnt, P.counters);
     }
 }
@@ -308,7 +311,7 @@ int resident_ctas(K kernel)
     return n < 1 ? 1 : n;
 }
 
-template <bool F, bool COUNT, bool CHK, int BX>
+template <bool F, bool COUNT, bool GEN, int BX>
 void launch_batch_shape(const PropGroup& tab, const JobList& J, int ctas_per_sm, int sms, int* next, cudaStream_t st)
 {
     const dim3 b(BX, PROP_THREADS / BX);
@@ -317,22 +320,22 @@ void launch_batch_shape(const PropGroup& tab, const JobList& J, int ctas_per_sm,
         const long long g = (long long)per_sm * sms;
         return (unsigned)(g < J.njobs ? g : J.njobs);
     };
-    k_prop_chain_b<F, COUNT, CHK, BX><<<grid(resident_ctas(k_prop_chain_b<F, COUNT, CHK, BX>)), b, 0, st>>>(
+    k_prop_chain_b<F, COUNT, GEN, BX><<<grid(resident_ctas(k_prop_chain_b<F, COUNT, GEN, BX>)), b, 0, st>>>(
         tab, J.jobs, J.njobs, next);
-    k_prop_klt_b<F, COUNT, CHK, BX><<<grid(resident_ctas(k_prop_klt_b<F, COUNT, CHK, BX>)), b, 0, st>>>(
+    k_prop_klt_b<F, COUNT, GEN, BX><<<grid(resident_ctas(k_prop_klt_b<F, COUNT, GEN, BX>)), b, 0, st>>>(
         tab, J.jobs, J.njobs, next + 1);
-    k_prop_final_b<F, COUNT, CHK, BX><<<grid(resident_ctas(k_prop_final_b<F, COUNT, CHK, BX>)), b, 0, st>>>(
+    k_prop_final_b<F, COUNT, GEN, BX><<<grid(resident_ctas(k_prop_final_b<F, COUNT, GEN, BX>)), b, 0, st>>>(
         tab, J.jobs, J.njobs, next + 2);
 }
 
 // the tile shapes of the batched kernels: 32 x 4 pixels (a warp = 32 pixels of a row) or
 // 16 x 8 (a warp = two rows of 16)
-template <bool F, bool COUNT, bool CHK>
+template <bool F, bool COUNT, bool GEN>
 void launch_batch_variant(const PropGroup& tab, const JobList& J, int tile_w, int ctas_per_sm, int sms, int* next,
                           cudaStream_t st)
 {
-    if (tile_w == 16) launch_batch_shape<F, COUNT, CHK, 16>(tab, J, ctas_per_sm, sms, next, st);
-    else launch_batch_shape<F, COUNT, CHK, 32>(tab, J, ctas_per_sm, sms, next, st);
+    if (tile_w == 16) launch_batch_shape<F, COUNT, GEN, 16>(tab, J, ctas_per_sm, sms, next, st);
+    else launch_batch_shape<F, COUNT, GEN, 32>(tab, J, ctas_per_sm, sms, next, st);
 }
 
 }  // namespace
@@ -366,7 +369,7 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
         sms = 1;
     }
     // as launch_propagate: uncounted passes run both variants (each table entry has dual = 1),
-    // counted ones the checked variant alone (dual = 0)
+    // counted ones the general variant alone (dual = 0)
     if (counting) {
         if (fused) launch_batch_variant<true, true, true>(tab, J, tile_w, ctas_per_sm, sms, next, st);
         else launch_batch_variant<false, true, true>(tab, J, tile_w, ctas_per_sm, sms, next, st);

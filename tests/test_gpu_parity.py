@@ -181,7 +181,7 @@ def test_kernels_fused_match_oracle(D, orc, case):
 
 
 def test_tiny_colours_take_exact_division(D, orc):
-    """Colour values below 2^-40 make the window loops run their checked variant (exact
+    """Colour values that are not k / 255 make the window loops run their general variant (with the exact
     division for truncated differences below 2^-100); results still equal the oracle's."""
     g = load_golden("lr_40x28")
     W, H, r, dmax, iters, pp, views = spec_of(g)
@@ -191,13 +191,73 @@ def test_tiny_colours_take_exact_division(D, orc):
     bwR[5:20, :, :3] *= tiny
     gL, gR, P = g["gL"], g["gR"], g["k_planes"]
     dL, dR, dgL, dgR, dP = (dev(D.t, a) for a in (bwL, bwR, gL, gR, P))
-    for f in (0, 1):   # both arithmetics launch the unchecked and the checked variant
+    for f in (0, 1):   # both arithmetics launch the pair-plane and the general variant
         for m in (1e10, 0.2):
             assert bits_equal(host(D.cost(dP, dL, dR, dgL, dgR, r, m, f)),
                               orc.cost(P, bwL, bwR, gL, gR, r, m, fused=f)).all()
         assert bits_equal(host(D.klt(dP, dL, dR, dgL, dgR, r, f)), orc.klt(P, bwL, bwR, gL, gR, r, fused=f)).all()
         init = host(D.init(dL, dR, dgL, dgR, r, dmax, 1, f))
         assert bits_equal(init, orc.init(bwL, bwR, gL, gR, r, dmax, 1, fused=f)).all()
+
+
+def pair_planes(rng, W, H, grad2):
+    """planes that meet the window loops' special cases: matched columns around both image borders, around
+    powers of two and at whole columns, tap weights at a sign change of the interpolated gradient, steep
+    and flat slopes, columns that overflow, NaN"""
+    P = np.zeros((H, W, 4), np.float32)
+    f = np.float32
+    for y in range(H):
+        for x in range(W):
+            kind = int(rng.integers(0, 8))
+            a, b = f(1.0), f(0.0)
+            if kind == 0:      # a whole or half column
+                c = f(rng.integers(-2 * W, 2 * W + 1)) * f(0.5)
+            elif kind == 1:    # just around a power of two
+                c = f(2.0 ** int(rng.integers(0, 10))) + f(rng.uniform(-1.6, 1.6)) - f(x)
+            elif kind == 2:    # the weight at which a gradient component changes sign, and its neighbours
+                k = int(rng.integers(0, W))
+                g0, g1 = grad2[y, k], grad2[y, min(k + 1, W - 1)]
+                j = int(rng.integers(0, 4))
+                t = g0[j] / (g0[j] - g1[j]) if g0[j] != g1[j] else f(0.25)
+                c = f(k) + f(t if 0 <= t < 1 else 0.5) - f(x)
+                for _ in range(int(rng.integers(0, 3))):
+                    c = np.nextafter(c, f(np.inf))
+            elif kind == 3:    # around the borders
+                c = (f(-1.0) if rng.random() < 0.5 else f(W)) - f(x) + f(rng.normal() * 2)
+            elif kind == 4:    # slanted
+                a, b = f(1 + rng.normal() * 0.3), f(rng.normal() * 0.3)
+                c = f(x) - a * f(x) - b * f(y) + f(rng.normal() * 3)
+            elif kind == 5:    # steep
+                a, b = f(rng.normal() * 30), f(rng.normal() * 30)
+                c = f(x) - a * f(x) - b * f(y)
+            elif kind == 6:    # just left of column 0
+                c = -f(x) - f(2.0) ** f(-int(rng.integers(1, 40)))
+            else:
+                a = f(rng.choice([1e6, 1e20, 1e35, -1e35, 3e38, np.inf, np.nan, 0.0, -1.0]))
+                b = f(rng.choice([0.0, 1e6, -1e35, 3e38]))
+                c = f(rng.choice([0.0, 1.0, -1e35, 1e38]))
+            P[y, x] = (a, b, c, rng.random())
+    return P
+
+
+@pytest.mark.parametrize("fused", [0, 1])
+@pytest.mark.parametrize("W,H,r", [(1, 1, 0), (2, 3, 1), (3, 2, 2), (33, 5, 0), (40, 9, 4), (131, 6, 3), (530, 4, 2),
+                                   (70, 12, 32)])
+def test_pair_plane_loops_match_oracle(D, orc, W, H, r, fused):
+    """The packed window loops against the oracle, bit for bit: images narrower than the window, even and odd row
+    lengths, and the planes of pair_planes; costs with and without an early exit and one Gauss-Newton step."""
+    rng = np.random.default_rng(1000 * W + r)
+    L = rng.integers(0, 256, (H, W, 4), dtype=np.uint8)
+    R = np.clip(L.astype(int) + rng.integers(-9, 10, L.shape), 0, 255).astype(np.uint8)
+    R[:, W // 2:W // 2 + 6] = 77   # equal texels: zero gradients of either sign
+    bwL, gL, _ = orc.prep(L, r, fused=fused)
+    bwR, gR, _ = orc.prep(R, r, fused=fused)
+    P = pair_planes(rng, W, H, gR)
+    dL, dR, dgL, dgR, dP = (dev(D.t, a) for a in (bwL, bwR, gL, gR, P))
+    for m in (1e10, 0.3, 0.0):
+        assert bits_equal(host(D.cost(dP, dL, dR, dgL, dgR, r, m, fused)),
+                          orc.cost(P, bwL, bwR, gL, gR, r, m, fused=fused)).all()
+    assert bits_equal(host(D.klt(dP, dL, dR, dgL, dgR, r, fused)), orc.klt(P, bwL, bwR, gL, gR, r, fused=fused)).all()
 
 
 def test_propagate_view_exchange_matches_oracle(D, orc):
