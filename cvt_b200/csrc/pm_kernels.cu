@@ -677,17 +677,17 @@ __device__ __forceinline__ bool unorm_byte(float v, uint32_t& k)
     return __float_as_uint((float)k / 255.0f) == __float_as_uint(v);
 }
 
-// The pair plane's sign threshold of one gradient component (PairRec): the smallest A in
-// [0, 2^15) for which the component interpolated at a = A 2^-15 has another sign than texel
-// i's, PAIR_NEVER if there is none.  Exact for weights between the grid points too: equal
-// signs interpolate to that sign for every a < 1; for opposite signs the two rounded products
-// grow and shrink monotonically in a, so the sign of their sum changes once.
+// The pair plane's sign word of one gradient component (PairRec).  Its threshold is the smallest A
+// in [0, 2^15) for which the component interpolated at a = A 2^-15 has another sign than texel i's,
+// 2^15 if there is none.  Exact for weights between the grid points too: equal signs
+// interpolate to that sign for every a < 1; for opposite signs the two rounded products grow
+// and shrink monotonically in a, so the sign of their sum changes once.
 template <bool F>
-__device__ __forceinline__ uint32_t pair_threshold(float g0, float g1)
+__device__ __forceinline__ uint32_t pair_sign_word(float g0, float g1)
 {
     const uint32_t s0 = __float_as_uint(g0) >> 31;
-    if (s0 == __float_as_uint(g1) >> 31) return PAIR_NEVER;
-    uint32_t lo = 0, hi = PAIR_NEVER;   // the answer lies in [lo, hi]
+    uint32_t lo = 0, hi = 0x8000u;   // the threshold lies in [lo, hi]
+    if (s0 == __float_as_uint(g1) >> 31) lo = hi;
 #pragma unroll 1
     while (lo < hi) {
         const uint32_t m = (lo + hi) >> 1;
@@ -696,7 +696,9 @@ __device__ __forceinline__ uint32_t pair_threshold(float g0, float g1)
         if (__float_as_uint(v) >> 31 != s0) hi = m;
         else lo = m + 1;
     }
-    return lo;
+    // positive texel i: bit 15 of A + 0x8000 - threshold is set from the threshold on; negative: bit 15 of
+    // A - threshold is set below it
+    return ((s0 ? 0u : 0x8000u) - lo) & 0xffffu;
 }
 
 // texel planes of one view (pm_window.cuh): column c in [-4, W+3] of the colour plane holds bw,
@@ -725,10 +727,10 @@ __global__ void k_pack_tex(float4* __restrict__ tex, const float4* __restrict__ 
     unorm_byte(col1.z, k[5]);
     ok &= fin(g.x) && fin(g.y) && fin(g.z) && fin(g.w);
     PairRec R;
-    R.x = k[0] | k[1] << 8 | k[2] << 16 | signbits4(g) << 24;
+    R.x = k[0] | k[1] << 8 | k[2] << 16;
     R.y = k[3] | k[4] << 8 | k[5] << 16;
-    R.z = pair_threshold<F>(g.y, g1.y) | pair_threshold<F>(g.w, g1.w) << 16;
-    R.w = pair_threshold<F>(g.x, g1.x) | pair_threshold<F>(g.z, g1.z) << 16;
+    R.z = pair_sign_word<F>(g.y, g1.y) | pair_sign_word<F>(g.w, g1.w) << 16;
+    R.w = pair_sign_word<F>(g.x, g1.x) | pair_sign_word<F>(g.z, g1.z) << 16;
     reinterpret_cast<PairRec*>(tex)[3 * plane + o] = R;
     if (c == s && !ok) atomicOr(reinterpret_cast<int*>(tex + TEX_PLANES * plane), 1);
 }

@@ -65,7 +65,7 @@ void prop_tile_shape(int* w, int* h);
 // false for any other width
 bool prop_batch_tile_shape(int tile_w, int* w, int* h);
 // pairs per batched propagate launch: their arguments are one kernel parameter block
-// (128 x 192 bytes, within the 32,764 bytes a launch may pass)
+// (128 x 184 bytes, within the 32,764 bytes a launch may pass)
 constexpr int PROP_GROUP = 128;
 struct PropGroup {
     PropParams p[PROP_GROUP];
@@ -149,7 +149,7 @@ inline ViewData make_view(const float4* t1, const float4* t2, int W, int H, int 
 {
     const int plane = tex_pitch(W) * H;
     return ViewData{t1, t2, W, H, r, tex_pitch(W), plane, reinterpret_cast<const int*>(t1 + (size_t)TEX_PLANES * plane),
-                    reinterpret_cast<const int*>(t2 + (size_t)TEX_PLANES * plane), make_float2(1.0f, 1.0f)};
+                    reinterpret_cast<const int*>(t2 + (size_t)TEX_PLANES * plane)};
 }
 void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, int fused, cudaStream_t st);
 // FP32 peak probe: `iters` rounds of independent fma chains per thread

@@ -28,23 +28,21 @@ namespace {
 #define PM_PROP_BY 4
 #endif
 constexpr int PROP_BX = PM_PROP_BX, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
-// Resident threads per SM asked of the register allocator for each kernel: 512 = 128 registers, which
-// the pair loops (two samples in flight per thread) use without spills.  Measured at 1280x720, r = 10, 3
-// iterations, ms (chain / Gauss-Newton): 512 threads 70.2 / 97.8, 640 (96 registers, 24-40 bytes
-// spilled) 70.6 / 100.8, 768 (80 registers, 64-190 bytes) 69.6 / 106.2; at 320x240 2.50 / 3.91, 2.81 /
-// 4.57, 2.82 / 4.91: the FMA pipe is busy at 16 warps already, and short grids gain from ILP.
-// The block shape does not matter (32x4 184.7 ms a call, 16x8 185.5, 8x16 187.4, 32x2 185.9).
+// Resident threads per SM asked of the register allocator for each kernel (640 = 96 registers, no
+// spills).  The window loops issue 88-92% of the cycles, so more threads give nothing: 1280x720,
+// r = 10, 3 iterations, ms (chain / Gauss-Newton): 512 threads 75.5 / 89.1, 640 69.2 / 88.9,
+// 768 69.2 / 88.7, 1024 (chain) 71.5; unrolling a row's loop by two 75.0 / 89.2 at 512.  The
+// block shape does not matter either (32x4, 16x8, 8x16 and 32x2 within 1.5% of each other).
 #ifndef PM_CHAIN_THREADS
-#define PM_CHAIN_THREADS 512
+#define PM_CHAIN_THREADS 640
 #endif
 #ifndef PM_KLT_THREADS
-#define PM_KLT_THREADS 512
+#define PM_KLT_THREADS 640
 #endif
 constexpr int PM_CHAIN_BLOCKS = PM_CHAIN_THREADS / PROP_THREADS, PM_KLT_BLOCKS = PM_KLT_THREADS / PROP_THREADS;
-// the batched (persistent) forms index each pair's arguments in a parameter block, which takes
-// registers; they are compiled for the same 128
+// the batched (persistent) forms index each pair's arguments in a parameter block, which takes registers
 #ifndef PM_BATCH_THREADS
-#define PM_BATCH_THREADS 512
+#define PM_BATCH_THREADS 640
 #endif
 constexpr int PM_BATCH_BLOCKS = PM_BATCH_THREADS / PROP_THREADS;
 

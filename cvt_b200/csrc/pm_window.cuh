@@ -22,12 +22,10 @@
 // threshold fixed by the two texels, so 4 x 16 bits replace 2 x 16 bytes and the four
 // interpolations.  3 gathers per Gauss-Newton sample and 1 per cost sample remain.
 //
-// Blackwell specifics: the bilinear colour mixes, the truncated absolute differences and
-// the Gauss-Newton sums run as packed FP32 pairs (sm_100), four gradient signs of a tap
-// are compared as 16-bit fields of two integer subtractions, and the three Gauss-Newton
-// taps at x'-1, x', x'+1 read three chained pair records.  Every packed operation rounds
-// per element exactly like its scalar form, so results equal the scalar restatement bit
-// for bit.
+// Arithmetic.  The pair loops are bound by instruction issue.  Packed FP32 instructions do
+// not help there: measured on B200, FFMA2 / FMUL2 / FADD2 hold the scheduler for 2 cycles (3 when all
+// three operands are register pairs), as two scalar instructions do, so the loops are scalar.
+// Every operation rounds as the scalar restatement does, so results equal it bit for bit.
 #pragma once
 
 #include "pm_device.cuh"
@@ -44,7 +42,6 @@ struct ViewData {
     int plane;                       // H * P
     const int* gen1;                 // the views' flags: read by the general loops (after the planes)
     const int* gen2;
-    float2 one;                      // (1, 1), opaque to the compiler (sum2)
     // colour texel (compact texel) of column 0 of row y
     __device__ __forceinline__ const float4* row1(int y) const { return t1 + (size_t)y * P + TEX_PAD; }
     __device__ __forceinline__ const float4* row1c(int y) const { return t1 + 2 * (size_t)plane + (size_t)y * P + TEX_PAD; }
@@ -54,14 +51,14 @@ struct ViewData {
 };
 
 // Pair record of columns (i, i + 1), one 16-byte word group:
-//   x  bytes r, g, b of texel i; bits 24-27 the signs of its four gradient components
+//   x  bytes r, g, b of texel i
 //   y  bytes r, g, b of texel i + 1
-//   z  sign thresholds of gradient components 1 (low half) and 3 (high half)
-//   w  sign thresholds of components 0 and 2
+//   z  sign words of gradient components 1 (low half) and 3 (high half)
+//   w  sign words of components 0 and 2
 // With A = a 2^15 the tap weight in units of 2^-15, the interpolated component has the sign
-// of texel i for A < threshold and the other sign from there on (pair_threshold).
+// of texel i for A < threshold and the other sign from there on (pair_sign_word); bit 15 of
+// A + sign word (mod 2^16) is that sign.
 typedef uint4 PairRec;
-constexpr uint32_t PAIR_NEVER = 0x8000u;   // threshold of a component whose sign does not change
 
 struct Counters {
     unsigned long long eval, klt, calls, exits;
@@ -426,91 +423,70 @@ __device__ __forceinline__ float4 klt2_general(const ViewData& V, int px, int py
 
 // ---- pair-plane loops ------------------------------------------------------------------
 
-// p + c per element, each rounded, for p a packed product.  A packed add fed by a packed multiply comes out
-// contracted (with .rn on both and with an fma by a literal 1 too); an fma by a kernel argument
-// that is 1 cannot.
-__device__ __forceinline__ float2 sum2(float2 p, float2 c, float2 one) { return __ffma2_rn(p, one, c); }
-
-// byte k of a record word, as the float byte * 2^-133: bits 16-23 of an otherwise zero word
-// (exponent field 0 or 1, one linear scale)
+// byte K of a record word / 255, correctly rounded, in one permute and one fma: the byte twice, in bits
+// 8-23 of an otherwise zero word, is x = 257 byte 2^-141 as a float (exponent field 0 or 1, one
+// linear scale).  RN(x RGB) for RGB = RN(2^141 / 65535) is RN(byte / 255) except where x RGB is
+// a tie, which rounds up in byte / 255 (its binary expansion goes on); the addend x, 2^125 times
+// smaller, decides the ties.  Equal to the division for all 256 bytes.
+#define PM_RGB 0x1.0001p+125f
 template <int K>
-__device__ __forceinline__ float pair_byte(uint32_t w)
+__device__ __forceinline__ float pair_unit(uint32_t w)
 {
-    return __uint_as_float(__byte_perm(w, 0u, 0x4044 | (K << 8)));
+    const float x = __uint_as_float(__byte_perm(w, 0u, 0x4004 | (K << 4) | (K << 8)));
+    return fmaf(x, PM_RGB, x);
 }
 
-// byte / 255 correctly rounded from byte * 2^-133: 2^133 / 255 = RGB_HI + RGB_LO and
-// RN(RGB_HI x + RN(RGB_LO x)) (the method of PM_D005; equal to the division for all 256 bytes)
-#define PM_RGB_HI 0x1.010102p+125f
-#define PM_RGB_LO -0x1.fdfdfep+100f
-__device__ __forceinline__ float2 rgb_unit(float2 x)
-{
-    return __ffma2_rn(x, f2(PM_RGB_HI, PM_RGB_HI), __fmul2_rn(x, f2(PM_RGB_LO, PM_RGB_LO)));
-}
-
-// bilinear mix of two texels' colours (rg0, b.x), (rg1, b.y) with weights (1 - a), a
+// T0 b1 + T1 a, the bilinear mix with b1 = 1 - a
 template <bool F>
-__device__ __forceinline__ void mix_rgb(float a, float b1, float2 rg0, float2 rg1, float2 b, float2& rg,
-                                        float& bl, float2 one)
+__device__ __forceinline__ float mix(float a, float b1, float t0, float t1)
 {
-    const float2 p0 = __fmul2_rn(f2(b1, b1), rg0);
-    if (F) {
-        rg = __ffma2_rn(f2(a, a), rg1, p0);
-        bl = fmaf(a, b.y, b1 * b.x);
-    } else {
-        rg = sum2(p0, __fmul2_rn(f2(a, a), rg1), one);
-        const float2 pb = __fmul2_rn(f2(b1, a), b);
-        bl = __fadd_rn(pb.x, pb.y);
-    }
+    return F ? fmaf(a, t1, b1 * t0) : b1 * t0 + a * t1;
 }
 
-// the interpolated colour of a tap from its pair record
-template <bool F>
-__device__ __forceinline__ void pair_rgb(const PairRec& R, float a, float2& rg, float& bl, float2 one)
+// fmin(|d|, 0.05) / 0.05 (ad_sum)
+__device__ __forceinline__ float trunc_ad(float d)
 {
-    const float2 rg0 = rgb_unit(f2(pair_byte<0>(R.x), pair_byte<1>(R.x)));
-    const float2 rg1 = rgb_unit(f2(pair_byte<0>(R.y), pair_byte<1>(R.y)));
-    mix_rgb<F>(a, 1.0f - a, rg0, rg1, rgb_unit(f2(pair_byte<2>(R.x), pair_byte<2>(R.y))), rg, bl, one);
+    const float m = fminf(fabsf(d), 0.05f);
+    return fmaf(m, 20.0f, m * PM_D005);
 }
 
-// ad_sum of an interpolated colour against minus the reference colour
-__device__ __forceinline__ float ad_pair(float2 rg, float bl, float2 nref_rg, float nref_b)
-{
-    const float2 d = __ffma2_rn(nref_rg, f2(1.0f, 1.0f), rg);
-    const float m2 = fminf(fabsf(bl + nref_b), 0.05f);
-    const float2 m = f2(fminf(fabsf(d.x), 0.05f), fminf(fabsf(d.y), 0.05f));
-    const float2 c = __ffma2_rn(m, f2(20.0f, 20.0f), __fmul2_rn(m, f2(PM_D005, PM_D005)));
-    return c.x + c.y + fmaf(m2, 20.0f, m2 * PM_D005);
-}
-
-// the tap weight 0 <= a < 1 as floor(a 2^15) with bit 15 set, in both halves of a word
+// the tap weight 0 <= a < 1 as floor(a 2^15) in both halves of a word
 __device__ __forceinline__ uint32_t pair_weight(float a)
 {
-    const uint32_t u = __float_as_uint(__fadd_rd(a, 257.0f));   // ulp(257) = 2^-15
+    const uint32_t u = __float_as_uint(__fadd_rd(a, 256.0f));   // ulp(256) = 2^-15
     return __byte_perm(u, u, 0x1010);
 }
 
-// The sign comparisons of a tap: each half of the differences has its bit 15 set when the weight has
-// reached the threshold (no half borrows: a half of M is >= 0x8000, a threshold <= 0x8000).  With the
-// weight rounded down and the threshold up, the answer is certain unless they differ by one
-// (a half equal to 0x7fff): sign_unsure.
+__device__ __forceinline__ uint32_t add_u16x2(uint32_t a, uint32_t b)
+{
+    uint32_t r;
+    asm("add.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// The signs of a tap's interpolated gradient.  With the weight rounded down and the threshold up to
+// multiples of 2^-15, a sign is certain unless weight + 1 = threshold, where the low 15 bits of its
+// half are all ones.
 struct PairSigns {
     uint32_t yw, xz;
 };
-__device__ __forceinline__ PairSigns pair_signs(uint32_t M, const PairRec& R) { return PairSigns{M - R.z, M - R.w}; }
-// max of the signed halves reaches 0x7fff: adding one to it changes its sign (a carry out of a low half
-// of -1 can only raise a high half, which at worst asks for the exact signs without need)
-__device__ __forceinline__ bool sign_unsure(uint32_t m) { return ((m + 0x00010001u) & ~m & 0x80008000u) != 0; }
-
-// number of gradient components whose sign differs from the first view's (sb1: sign_bytes)
-__device__ __forceinline__ int pair_mismatch(const PairSigns& d, uint32_t w0, uint32_t sb1)
+__device__ __forceinline__ PairSigns pair_signs(uint32_t A, const PairRec& R)
 {
-    const uint32_t flips = __byte_perm(d.xz, d.yw, 0x7351);          // component c's flag at bit 8 c + 7
-    const uint32_t s0 = (w0 >> 24) * 0x10204080u;                    // bit c of the four signs to bit 8 c + 7
-    return __popc((flips ^ s0 ^ sb1) & 0x80808080u);
+    return PairSigns{add_u16x2(A, R.z), add_u16x2(A, R.w)};
 }
+// number of components whose sign differs from the first view's (sb1: sign_bytes)
+__device__ __forceinline__ int pair_mismatch(const PairSigns& d, uint32_t sb1)
+{
+    return __popc((__byte_perm(d.xz, d.yw, 0x7351) ^ sb1) & 0x80808080u);
+}
+// the largest half so far, each with its bit 15 set: 0xffff when some sign was unsure
+__device__ __forceinline__ uint32_t unsure_max(uint32_t m, const PairSigns& d)
+{
+    return __vmaxu2(m, __vmaxu2(d.yw | 0x80008000u, d.xz | 0x80008000u));
+}
+__device__ __forceinline__ bool unsure(uint32_t m) { return (m >> 16) == 0xffffu || (m & 0xffffu) == 0xffffu; }
 
-// the same from the interpolated gradient itself (g: gradient texel i)
+// the number of mismatches from the interpolated gradient itself (g: gradient texel i)
 template <bool F>
 __device__ __forceinline__ int exact_mismatch(const float4* __restrict__ g, float a, uint32_t sb1)
 {
@@ -520,126 +496,54 @@ __device__ __forceinline__ int exact_mismatch(const float4* __restrict__ g, floa
     return sign_mismatch(sb1, sign_bytes(make_float4(u.x, u.y, v.x, v.y)));
 }
 
-// support_weight of two samples
+// the matched column s.x qx + s.y qy + s.z (byq = s.y qy)
 template <bool F>
-__device__ __forceinline__ float2 support_weight2(float2 dx, float2 dy, float2 dz, float2 one)
+__device__ __forceinline__ float match(float4 s, float qx, float byq)
 {
-    const float2 wr = f2(PM_GW_R, PM_GW_R), wg = f2(PM_GW_G, PM_GW_G), wb = f2(PM_GW_B, PM_GW_B);
-    float2 g;
-    if (F) g = __ffma2_rn(dz, wb, __ffma2_rn(dy, wg, __fmul2_rn(dx, wr)));
-    else g = sum2(__fmul2_rn(dz, wb), sum2(__fmul2_rn(dy, wg), __fmul2_rn(dx, wr), one), one);
-    const float2 x = f2(-fabsf(g.x) * 12.0f, -fabsf(g.y) * 12.0f);
-    // expf_neg, element by element
-    const float M = 12582912.0f;
-    const float2 t = sum2(__fmul2_rn(x, f2(1.44269502162933349609375f, 1.44269502162933349609375f)), f2(M, M), one);
-    const float2 n = __fadd2_rn(t, f2(-M, -M));
-    float2 r = __ffma2_rn(n, f2(-0.693145751953125f, -0.693145751953125f), x);
-    r = __ffma2_rn(n, f2(-1.428606765330187045e-06f, -1.428606765330187045e-06f), r);
-    float2 p = f2(1.9841270113829523e-4f, 1.9841270113829523e-4f);
-    p = __ffma2_rn(p, r, f2(1.3888889e-3f, 1.3888889e-3f));
-    p = __ffma2_rn(p, r, f2(8.3333338e-3f, 8.3333338e-3f));
-    p = __ffma2_rn(p, r, f2(4.1666668e-2f, 4.1666668e-2f));
-    p = __ffma2_rn(p, r, f2(1.6666667e-1f, 1.6666667e-1f));
-    p = __ffma2_rn(p, r, f2(0.5f, 0.5f));
-    p = __ffma2_rn(p, r, f2(1.0f, 1.0f));
-    p = __ffma2_rn(p, r, f2(1.0f, 1.0f));
-    return f2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)),
-              __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
+    return F ? fmaf(s.x, qx, byq) + s.z : s.x * qx + byq + s.z;
 }
 
-// the matched columns s.x * qx + s.y * qy + s.z of two samples (byq = s.y * qy)
+// One sample of patch_eval_census (:690-722): compact texel q of the first view, matched column p2x whose
+// t = (p2x + 0.5) - 0.5 lies in [0, W], weight w.  The column's texel is at base + 16 * (bits of the float
+// 2^23 + column).  Returns the sample's cost and the signs.
 template <bool F>
-__device__ __forceinline__ float2 match2(float4 s, float2 qx, float byq, float2 one)
+__device__ __forceinline__ float eval_sample_pair(uintptr_t base, float4 q, float t, PairSigns& d, float& a)
 {
-    const float2 sx = f2(s.x, s.x), by = f2(byq, byq), sz = f2(s.z, s.z);
-    return __fadd2_rn(F ? __ffma2_rn(sx, qx, by) : sum2(__fmul2_rn(sx, qx), by, one), sz);
-}
-
-// one colour channel (byte K of two words each) of two samples mixed with weights b1 = 1 - a, a
-template <bool F, int K>
-__device__ __forceinline__ float2 mix_channel2(uint32_t w0, uint32_t w1, uint32_t v0, uint32_t v1, float2 a, float2 b1, float2 one)
-{
-    const float2 c0 = rgb_unit(f2(pair_byte<K>(w0), pair_byte<K>(w1))), c1 = rgb_unit(f2(pair_byte<K>(v0), pair_byte<K>(v1)));
-    const float2 p0 = __fmul2_rn(b1, c0);
-    return F ? __ffma2_rn(a, c1, p0) : sum2(__fmul2_rn(a, c1), p0, one);
-}
-
-// fmin(|d|, 0.05) / 0.05 of two samples (ad_sum)
-__device__ __forceinline__ float2 trunc2(float2 d)
-{
-    const float2 m = f2(fminf(fabsf(d.x), 0.05f), fminf(fabsf(d.y), 0.05f));
-    return __ffma2_rn(m, f2(20.0f, 20.0f), __fmul2_rn(m, f2(PM_D005, PM_D005)));
-}
-
-// one window sample of patch_eval_census at (qx, row of q1) whose matched column p2x lies in the image
-template <bool F>
-__device__ __forceinline__ void eval_one(const ViewData& V, uintptr_t base, const float4* __restrict__ g2, float4 q,
-                                         float4 in, float p2x, float& census, float& wsum)
-{
-    const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
-    // 0 <= t <= W: the floor is the integer part of t + 2^23 rounded down
-    const float t = (p2x + 0.5f) - 0.5f;
-    const float fm = __fadd_rd(t, 8388608.0f);
-    const float a = t - (fm - 8388608.0f);
+    const float fm = __fadd_rd(t, 8388608.0f);   // 2^23 + floor(t)
+    a = t - (fm - 8388608.0f);
     const PairRec R = __ldg(reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fm) * 16u));
-    const PairSigns d = pair_signs(pair_weight(a), R);
-    int nm = pair_mismatch(d, R.x, __float_as_uint(q.w));
-    if (sign_unsure(__vmaxs2(d.yw, d.xz)))
-        nm = exact_mismatch<F>(g2 + (__float_as_int(fm) - 0x4B000000), a, __float_as_uint(q.w));
-    float2 rg;
-    float bl;
-    pair_rgb<F>(R, a, rg, bl, V.one);
-    // cost + 0.875f * (0.25f * n): the product 0.21875 n is exact, so one fma rounds the same
-    const float cost = fmaf(0.21875f, (float)nm, PM_K033_8 * ad_pair(rg, bl, f2(-q.x, -q.y), -q.z));
-    census = F ? fmaf(w, cost, census) : census + w * cost;
-    wsum += w;
+    d = pair_signs(pair_weight(a), R);
+    const float b1 = 1.0f - a;
+    float ad = trunc_ad(mix<F>(a, b1, pair_unit<0>(R.x), pair_unit<0>(R.y)) - q.x);
+    ad = ad + trunc_ad(mix<F>(a, b1, pair_unit<1>(R.x), pair_unit<1>(R.y)) - q.y);
+    ad = ad + trunc_ad(mix<F>(a, b1, pair_unit<2>(R.x), pair_unit<2>(R.y)) - q.z);
+    return PM_K033_8 * ad;
 }
 
-// a row of patch_eval_pair, two samples per packed instruction; IN: every matched column, one past
-// the end included, lies in the image (otherwise: is finite; samples outside get weight 0).
-// Returns the maximum of the sign comparisons for sign_unsure.
-template <bool F, bool IN>
-__device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, float2 one, uintptr_t base,
-                                             const float4* __restrict__ q1, float4 in, float4 s, float byq, float qx0,
-                                             float qx1, float fW)
+// a row of patch_eval_pair.  IN: every matched column lies in the image; otherwise all are finite and
+// samples outside get weight 0.  SURE: no sign can be unsure; otherwise returns unsure_max.
+template <bool F, bool IN, bool SURE>
+__device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, uintptr_t base, const float4* __restrict__ q1,
+                                             float4 in, float4 s, float byq, float qx0, float qx1, float fW)
 {
-    uint32_t sure = 0x80008000u;
-    for (float2 qx = f2(qx0, qx0 + 1.0f); qx.x <= qx1; qx = __fadd2_rn(qx, f2(2.0f, 2.0f)), q1 += 2) {
-        const float4 q0 = __ldg(q1), qn = __ldg(q1 + 1);
-        const float2 p = match2<F>(s, qx, byq, one);
-        float2 t = __fadd2_rn(__fadd2_rn(p, f2(0.5f, 0.5f)), f2(-0.5f, -0.5f));
-        if (!IN) t = f2(fminf(fmaxf(t.x, 0.0f), fW), fminf(fmaxf(t.y, 0.0f), fW));
-        // 0 <= t <= W: the floor is the integer part of t + 2^23 rounded down
-        const float2 fm = __fadd2_rd(t, f2(8388608.0f, 8388608.0f));
-        const PairRec R0 = __ldg(reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fm.x) * 16u));
-        const PairRec R1 = __ldg(reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fm.y) * 16u));
-        const float2 a = __ffma2_rn(__fadd2_rn(fm, f2(-8388608.0f, -8388608.0f)), f2(-1.0f, -1.0f), t);
-        const float2 b1 = __ffma2_rn(a, f2(-1.0f, -1.0f), f2(1.0f, 1.0f));
-        float2 w = support_weight2<F>(f2(q0.x - in.x, qn.x - in.x), f2(q0.y - in.y, qn.y - in.y),
-                                      f2(q0.z - in.z, qn.z - in.z), one);
-        if (!IN && !(p.x >= 0.0f && p.x < fW)) w.x = 0.0f;
-        if (!(qx.y <= qx1 && (IN || (p.y >= 0.0f && p.y < fW)))) w.y = 0.0f;   // an odd row's last pair has one sample
-        const PairSigns d0 = pair_signs(pair_weight(a.x), R0), d1 = pair_signs(pair_weight(a.y), R1);
-        sure = __vimax3_s16x2(__vimax3_s16x2(sure, d0.yw, d0.xz), d1.yw, d1.xz);
-        const float2 nm = f2((float)pair_mismatch(d0, R0.x, __float_as_uint(q0.w)),
-                             (float)pair_mismatch(d1, R1.x, __float_as_uint(qn.w)));
-        float2 v = mix_channel2<F, 0>(R0.x, R1.x, R0.y, R1.y, a, b1, one);
-        float2 ad = trunc2(f2(v.x - q0.x, v.y - qn.x));
-        v = mix_channel2<F, 1>(R0.x, R1.x, R0.y, R1.y, a, b1, one);
-        ad = __fadd2_rn(ad, trunc2(f2(v.x - q0.y, v.y - qn.y)));
-        v = mix_channel2<F, 2>(R0.x, R1.x, R0.y, R1.y, a, b1, one);
-        ad = __fadd2_rn(ad, trunc2(f2(v.x - q0.z, v.y - qn.z)));
+    uint32_t m = 0;
+    for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
+        const float4 q = __ldg(q1);
+        const float p2x = match<F>(s, qx, byq);
+        float t = (p2x + 0.5f) - 0.5f;
+        if (!IN) t = fminf(fmaxf(t, 0.0f), fW);
+        float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
+        if (!IN) w = p2x >= 0.0f && p2x < fW ? w : 0.0f;
+        PairSigns d;
+        float a;
+        float cost = eval_sample_pair<F>(base, q, t, d, a);
+        if (!SURE) m = unsure_max(m, d);
         // cost + 0.875f * (0.25f * n): the product 0.21875 n is exact, so one fma rounds the same
-        const float2 cost = __ffma2_rn(f2(0.21875f, 0.21875f), nm, __fmul2_rn(f2(PM_K033_8, PM_K033_8), ad));
-        if (F) {
-            census = fmaf(w.y, cost.y, fmaf(w.x, cost.x, census));
-        } else {
-            const float2 wc = __fmul2_rn(w, cost);
-            census = __fadd_rn(__fadd_rn(census, wc.x), wc.y);
-        }
-        wsum = (wsum + w.x) + w.y;
+        cost = fmaf(0.21875f, (float)pair_mismatch(d, __float_as_uint(q.w)), cost);
+        census = F ? fmaf(w, cost, census) : census + w * cost;
+        wsum += w;
     }
-    return sure;
+    return m;
 }
 
 // patch_eval_census (:661-736) over pair records.
@@ -648,17 +552,16 @@ __device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, float2 
 // `census / bilw >= mincost` with a sample counted (:724), is decided by the census at the row's
 // end; it is tested there as census >= exit_threshold(mincost, bilw).
 //
-// Rows run two samples per packed instruction; p2x is monotone along a row, so its two ends decide for
-// the warp whether samples can lie outside the image, or a column can be non-finite.  Such
-// rows, and rows where some sign was unsure, run sample by sample.  From column 256 on a tap
-// weight is a multiple of 2^-15 and no sign is unsure.
+// p2x is monotone along a row, so its two ends decide, for the warp, whether samples can lie outside
+// the image or a column be non-finite.  From column 256 on a tap weight is a multiple of
+// 2^-15 and no sign is unsure.  Rows with a non-finite column and rows where some sign was
+// unsure run sample by sample with the signs from the gradients.
 template <bool F>
 __device__ __forceinline__ float patch_eval_pair(const ViewData& V, int px, int py, float4 s, float mincost)
 {
     const float cx = (float)px, cy = (float)py;
     if (!plane_usable(s, cx, cy, V.W)) return 1e5f;
     const int W = V.W;
-    const float2 one = V.one;
     const float4 in = __ldg(V.row1(py) + px);
     const float thr = exit_threshold(mincost, in.w);
     float wsum = 0.0f, census = 0.0f;
@@ -671,36 +574,44 @@ __device__ __forceinline__ float patch_eval_pair(const ViewData& V, int px, int 
     for (int iy = py + dy0; iy <= py + dy1; iy++, qy += 1.0f) {
         const float byq = s.y * qy;
         const float4* __restrict__ q1 = V.row1c(iy) + px + dx0;
-        // column c of the row is at base + 16 * (bits of the float 2^23 + c)
         const uintptr_t base = reinterpret_cast<uintptr_t>(V.row2p(iy)) - (uintptr_t)0x4B000000u * 16u;
-        const float2 pe = match2<F>(s, f2(qx0, qx1 + 1.0f), byq, one);
-        const float plo = fminf(pe.x, pe.y);
+        const float pa = match<F>(s, qx0, byq), pb = match<F>(s, qx1, byq);
+        const float plo = fminf(pa, pb), phi = fmaxf(pa, pb);
         const float census0 = census, wsum0 = wsum;
-        const bool finite = fin(pe.x) && fin(pe.y);
+        const bool in_image = pa >= 0.0f && pb >= 0.0f && phi < fW;
+        const bool sure = in_image && plo >= 256.0f;
         const unsigned lanes = __activemask();
         bool single = true;
-        if (__all_sync(lanes, pe.x >= 0.0f && pe.y >= 0.0f && pe.x < fW && pe.y < fW)) {
-            single = sign_unsure(eval_row<F, true>(census, wsum, one, base, q1, in, s, byq, qx0, qx1, fW)) && plo < 256.0f;
-        } else if (__all_sync(lanes, finite)) {
-            if (!__any_sync(lanes, plo < fW && fmaxf(pe.x, pe.y) >= 0.0f)) continue;
-            single = sign_unsure(eval_row<F, false>(census, wsum, one, base, q1, in, s, byq, qx0, qx1, fW)) && plo < 256.0f;
+        if (__all_sync(lanes, sure)) {
+            eval_row<F, true, true>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW);
+            single = false;
+        } else if (__all_sync(lanes, in_image)) {
+            single = unsure(eval_row<F, true, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
+        } else if (__all_sync(lanes, fin(pa) && fin(pb))) {
+            if (!__any_sync(lanes, plo < fW && phi >= 0.0f)) continue;
+            single = unsure(eval_row<F, false, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
         }
         if (single) {
             census = census0;
             wsum = wsum0;
             const float4* __restrict__ g2 = V.row2(iy) + V.plane;
             for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
-                const float p2x = F ? fmaf(s.x, qx, byq) + s.z : s.x * qx + byq + s.z;
+                const float p2x = match<F>(s, qx, byq);
                 if (p2x < 0 || p2x >= fW) continue;
-                const float4 q = __ldg(q1);   // compact texel
+                const float4 q = __ldg(q1);
+                const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
+                float cost;
                 if (p2x == p2x) {
-                    eval_one<F>(V, base, g2, q, in, p2x, census, wsum);
+                    PairSigns d;
+                    float a;
+                    const float t = (p2x + 0.5f) - 0.5f;
+                    cost = eval_sample_pair<F>(base, q, t, d, a);
+                    cost = fmaf(0.21875f, (float)exact_mismatch<F>(g2 + (int)t, a, __float_as_uint(q.w)), cost);
                 } else {   // a NaN column reads the positive quiet NaN: full colour cost, positive signs
-                    const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
-                    const float cost = fmaf(0.21875f, (float)sign_mismatch(__float_as_uint(q.w), 0u), PM_K033_8 * 3.0f);
-                    census = F ? fmaf(w, cost, census) : census + w * cost;
-                    wsum += w;
+                    cost = fmaf(0.21875f, (float)sign_mismatch(__float_as_uint(q.w), 0u), PM_K033_8 * 3.0f);
                 }
+                census = F ? fmaf(w, cost, census) : census + w * cost;
+                wsum += w;
             }
         }
         if (census >= thr && wsum > 0.0f) return 1.0f;
@@ -724,143 +635,147 @@ struct KltSums {
     float J0, J1, J2, h00, h01, h02, h11, h12, h22;
 };
 
-// sum + v.x * f.x, then + v.y * f.y
+// the colour cost of a tap: texels t0, t1 (r, g, b) mixed with weights b1 = 1 - a, a, against minus the
+// reference colour
 template <bool F>
-__device__ __forceinline__ float accum2(float sum, float2 v, float2 f)
+__device__ __forceinline__ float tap_ad(float3 t0, float3 t1, float a, float b1, float3 nref)
 {
-    if (F) return fmaf(v.y, f.y, fmaf(v.x, f.x, sum));
-    const float2 p = __fmul2_rn(v, f);
-    return __fadd_rn(__fadd_rn(sum, p.x), p.y);
+    const float c0 = trunc_ad(mix<F>(a, b1, t0.x, t1.x) + nref.x), c1 = trunc_ad(mix<F>(a, b1, t0.y, t1.y) + nref.y),
+                c2 = trunc_ad(mix<F>(a, b1, t0.z, t1.z) + nref.z);
+    return c0 + c1 + c2;
 }
 
-// the costs of one tap of two samples: colour bytes of the texels on its left (l0, l1) and right (r0, r1)
+__device__ __forceinline__ float3 pair_rgb(uint32_t w) { return make_float3(pair_unit<0>(w), pair_unit<1>(w), pair_unit<2>(w)); }
+
+// one tap on its own: the coordinate u + 0.5 and its floor as the source forms them, the column
+// clamped to the padded row, where the records hold the edge texels that the source's clamp
+// gives, the signs from the gradients themselves (row2, g2: column 0 of the rows)
 template <bool F>
-__device__ __forceinline__ float2 tap2(uint32_t l0, uint32_t l1, uint32_t r0, uint32_t r1, float2 a, float2 b1, float2 nr,
-                                       float2 ng, float2 nb, float2 k1, float2 x, int n0, int n1, float2 one)
+__device__ __forceinline__ float tap_alone(float u, int W, const float4* __restrict__ row2, const float4* __restrict__ g2,
+                                           float3 nref, uint32_t sb1, float k1, float x)
 {
-    float2 ad = trunc2(__fadd2_rn(mix_channel2<F, 0>(l0, l1, r0, r1, a, b1, one), nr));
-    ad = __fadd2_rn(ad, trunc2(__fadd2_rn(mix_channel2<F, 1>(l0, l1, r0, r1, a, b1, one), ng)));
-    ad = __fadd2_rn(ad, trunc2(__fadd2_rn(mix_channel2<F, 2>(l0, l1, r0, r1, a, b1, one), nb)));
-    return __ffma2_rn(x, f2((float)n0, (float)n1), __fmul2_rn(k1, ad));
+    const float t = (u + 0.5f) - 0.5f;
+    const float fl = floorf(t);
+    const float a = t - fl;
+    const int c = (int)fminf(fmaxf(fl, -2.0f), (float)W);
+    const PairRec R = __ldg(reinterpret_cast<const uint4*>(row2 + c));
+    return tap_cost(k1, x, tap_ad<F>(pair_rgb(R.x), pair_rgb(R.y), a, 1.0f - a, nref), exact_mismatch<F>(g2 + c, a, sb1));
 }
 
-// one tap of two samples on its own: the coordinate u + 0.5 and its floor as the source forms them, the
-// column clamped to the padded row, where the records hold the edge texels that the source's
-// clamp gives, the signs from the gradients themselves
-template <bool F>
-__device__ __forceinline__ float2 tap_alone2(float2 u, const ViewData& V, const float4* __restrict__ row2,
-                                             const float4* __restrict__ g2, float2 nr, float2 ng, float2 nb, uint32_t s0,
-                                             uint32_t sn, float2 k1, float2 x)
+// A row of klt2_pair (row2, g2: column 0 of the pair and gradient rows).
+// EVEN: every p2x is at least 1 with p2x + 1.5 in the same binade, below 2^22.  p2x is then a
+// multiple of its ulp <= 0.5, the +-1 and +-0.5 of the source are exact, and the taps at t - 1, t,
+// t + 1 share the weight p2x - floor(p2x).  Otherwise each tap's coordinate is formed as the source
+// forms it; mostly the floors are still f - 1, f, f + 1 and only the weights differ in the last bit, and the
+// weights decide whether that holds: t - f is in [0, 1) exactly if f is t's floor.
+// The three taps read three consecutive records, whose four texels are decoded once.  The column f
+// is clamped to the padded row, where records beyond the image hold edge texels, as the
+// source's clamp gives.  Where a weight is out of range (floors that do not chain, a non-finite column) or,
+// not SURE, a sign unsure, each tap is read on its own.
+template <bool F, bool EVEN, bool SURE>
+__device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restrict__ row2, const float4* __restrict__ g2,
+                                        const float4* __restrict__ q1, float4 c1, float4 s, float byq, float qx0, float qx1,
+                                        float qy)
 {
-    const float2 t = __fadd2_rn(__fadd2_rn(u, f2(0.5f, 0.5f)), f2(-0.5f, -0.5f));
-    const float2 fl = f2(floorf(t.x), floorf(t.y));
-    const float2 a = __ffma2_rn(fl, f2(-1.0f, -1.0f), t);
-    const float2 b1 = __ffma2_rn(a, f2(-1.0f, -1.0f), f2(1.0f, 1.0f));
-    const float fW = (float)V.W;
-    const int c0 = (int)fminf(fmaxf(fl.x, -2.0f), fW), cn = (int)fminf(fmaxf(fl.y, -2.0f), fW);
-    const uint4* row = reinterpret_cast<const uint4*>(row2);
-    const PairRec A = __ldg(row + c0), B = __ldg(row + cn);
-    return tap2<F>(A.x, B.x, A.y, B.y, a, b1, nr, ng, nb, k1, x, exact_mismatch<F>(g2 + c0, a.x, s0),
-                   exact_mismatch<F>(g2 + cn, a.y, sn), V.one);
+    const float MAGIC = EVEN ? 8388608.0f : 12582912.0f;   // MAGIC + t rounded down: MAGIC + floor(t), t >= 0 or |t| < 2^22
+    // column c of the row is at base + 16 * (bits of the float MAGIC + c)
+    const uintptr_t base = reinterpret_cast<uintptr_t>(row2) - (uintptr_t)(EVEN ? 0x4B000000u : 0x4B400000u) * 16u;
+    const float first = MAGIC - 3.0f, last = MAGIC + (float)(W + 1);
+    const float yy = qy * qy;
+    for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
+        const float4 q = __ldg(q1);
+        const float p2x = match<F>(s, qx, byq);
+        const float t0 = EVEN ? p2x : (p2x + 0.5f) - 0.5f;
+        const float fm = __fadd_rd(t0, MAGIC);
+        const float fc = EVEN ? fminf(fm, last) : fminf(fmaxf(fm, first), last);
+        const uint4* b = reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fc) * 16u);
+        const PairRec Rm = __ldg(b - 1), R0 = __ldg(b), Rp = __ldg(b + 1);
+        const float f = fm - MAGIC;
+        const float a0 = t0 - f;
+        float am = a0, ap = a0;
+        if (!EVEN) {
+            am = (((p2x + -1.0f) + 0.5f) - 0.5f) - (f - 1.0f);
+            ap = (((p2x + 1.0f) + 0.5f) - 0.5f) - (f + 1.0f);
+        }
+        const uint32_t A0 = pair_weight(a0), Am = EVEN ? A0 : pair_weight(am), Ap = EVEN ? A0 : pair_weight(ap);
+        const uint32_t sb1 = __float_as_uint(q.w);
+        const PairSigns dm = pair_signs(Am, Rm), d0 = pair_signs(A0, R0), dp = pair_signs(Ap, Rp);
+        const float3 nref = make_float3(c1.x - q.x, c1.y - q.y, c1.z - q.z);   // minus the colour difference
+        float w1 = support_weight<F>(nref.x, nref.y, nref.z);
+        const float k1 = w1 * PM_K033_8, x = w1 * 0.21875f;   // (w1 * 0.875f) * 0.25, exact scaling
+        const float b0 = 1.0f - a0, bm = EVEN ? b0 : 1.0f - am, bp = EVEN ? b0 : 1.0f - ap;
+        const float3 tA = pair_rgb(Rm.x), tB = pair_rgb(R0.x);
+        float Cm = tap_cost(k1, x, tap_ad<F>(tA, tB, am, bm, nref), pair_mismatch(dm, sb1));
+        const float3 tC = pair_rgb(R0.y);
+        float C = tap_cost(k1, x, tap_ad<F>(tB, tC, a0, b0, nref), pair_mismatch(d0, sb1));
+        const float3 tD = pair_rgb(Rp.y);
+        float Cp = tap_cost(k1, x, tap_ad<F>(tC, tD, ap, bp, nref), pair_mismatch(dp, sb1));
+        bool alone = false;
+        if (!SURE) alone = unsure(unsure_max(unsure_max(unsure_max(0u, dm), d0), dp));
+        // a weight in [0, 1) has bits below 1.0f's; a negative one or a NaN has not
+        if (!EVEN) alone |= max(max(__float_as_uint(am), __float_as_uint(a0)), __float_as_uint(ap)) >= 0x3f800000u;
+        if (alone) {
+            Cm = tap_alone<F>(p2x + -1.0f, W, row2, g2, nref, sb1, k1, x);
+            C = tap_alone<F>(p2x, W, row2, g2, nref, sb1, k1, x);
+            Cp = tap_alone<F>(p2x + 1.0f, W, row2, g2, nref, sb1, k1, x);
+            // a non-finite column reads NaN texels for all three taps: equal costs, nothing added
+            if (!fin(p2x)) w1 = Cm = C = Cp = 0.0f;
+        }
+        // the update of :394-402 without a branch (KltSums)
+        const float curv = fmaf(-2.0f, C, Cp + Cm);   // 2 C is exact
+        const float wt = curv > 0.0f ? w1 : 0.0f;
+        const float t = wt * (Cm - Cp), sc = wt * curv;
+        if (F) {
+            A.J0 = fmaf(t, qx, A.J0);
+            A.J1 = fmaf(t, qy, A.J1);
+            A.h00 = fmaf(sc, qx * qx, A.h00);
+            A.h01 = fmaf(sc, qx * qy, A.h01);
+            A.h02 = fmaf(sc, qx, A.h02);
+            A.h11 = fmaf(sc, yy, A.h11);
+            A.h12 = fmaf(sc, qy, A.h12);
+        } else {
+            A.J0 = A.J0 + t * qx;
+            A.J1 = A.J1 + t * qy;
+            A.h00 = A.h00 + sc * (qx * qx);
+            A.h01 = A.h01 + sc * (qx * qy);
+            A.h02 = A.h02 + sc * qx;
+            A.h11 = A.h11 + sc * yy;
+            A.h12 = A.h12 + sc * qy;
+        }
+        A.J2 = A.J2 + t;
+        A.h22 = A.h22 + sc;
+    }
 }
 
-// patch_census_klt2 (:326-410) over pair records, two samples of a row per packed instruction.
-//
-// The three taps at t - 1, t, t + 1 (each coordinate formed as the source forms it) mostly have the floors
-// f - 1, f, f + 1: they then read three consecutive records, whose four texels are decoded once,
-// each with its own weight (the weights differ in the last bit near powers of two).  The weights decide
-// whether that holds: t - f in [0, 1) exactly if f is t's floor.  The column f is clamped
-// to the padded row, where records beyond the image hold edge texels, as the source's clamp gives.
-// Where a weight is out of range (floors that do not chain, a non-finite column) or a sign unsure, each
-// tap of the pair is read on its own.
+// patch_census_klt2 (:326-410) over pair records.  p2x is monotone along a row, so its two ends decide
+// the row's kind (klt_row), for the warp: one whose lanes differ would run several loops.
 template <bool F>
 __device__ __forceinline__ float4 klt2_pair(const ViewData& V, int px, int py, float4 s)
 {
     // a NaN plane has no column: no sample counts, the 0 / 0 solution is NaN
     if (s.x != s.x || s.y != s.y || s.z != s.z) return f4(qnan(), qnan(), qnan(), s.w - 1e5f);
     const float cxf = (float)px, cyf = (float)py;
-    const float2 one = V.one;
     KltSums A = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     const float4 c1 = __ldg(V.row1(py) + px);
     const int r = V.r;
     const int dy0 = max(-r, -py), dy1 = min(r, V.H - 1 - py);
     const int dx0 = max(-r, 1 - px), dx1 = min(r, V.W - 2 - px);   // the 3-point cost needs 1 <= qx < W - 1
     const float qx0 = cxf + (float)dx0, qx1 = cxf + (float)dx1;
-    const float MAGIC = 12582912.0f;   // 1.5 * 2^23: MAGIC + t rounded down is MAGIC + floor(t) for |t| < 2^22
-    const float first = MAGIC - 3.0f, last = MAGIC + (float)(V.W + 1);
     float qy = cyf + (float)dy0;
     for (int iy = py + dy0; iy <= py + dy1; iy++, qy += 1.0f) {
         const float byq = s.y * qy;
         const float4* __restrict__ q1 = V.row1c(iy) + px + dx0;
-        // column c of the row is at base + 16 * (bits of the float MAGIC + c)
-        const uintptr_t base = reinterpret_cast<uintptr_t>(V.row2p(iy)) - (uintptr_t)0x4B400000u * 16u;
-        for (float2 qx = f2(qx0, qx0 + 1.0f); qx.x <= qx1; qx = __fadd2_rn(qx, f2(2.0f, 2.0f)), q1 += 2) {
-            const float4 q0 = __ldg(q1), qn = __ldg(q1 + 1);
-            const float2 p = match2<F>(s, qx, byq, one);
-            const float2 h = f2(0.5f, 0.5f), mh = f2(-0.5f, -0.5f);
-            const float2 t0 = __fadd2_rn(__fadd2_rn(p, h), mh);
-            const float2 tm = __fadd2_rn(__fadd2_rn(__fadd2_rn(p, f2(-1.0f, -1.0f)), h), mh);
-            const float2 tp = __fadd2_rn(__fadd2_rn(__fadd2_rn(p, f2(1.0f, 1.0f)), h), mh);
-            const float2 fm = __fadd2_rd(t0, f2(MAGIC, MAGIC));
-            const uint4* b0 =
-                reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fminf(fmaxf(fm.x, first), last)) * 16u);
-            const uint4* bn =
-                reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fminf(fmaxf(fm.y, first), last)) * 16u);
-            const PairRec Am = __ldg(b0 - 1), A0 = __ldg(b0), Ap = __ldg(b0 + 1);
-            const PairRec Bm = __ldg(bn - 1), B0 = __ldg(bn), Bp = __ldg(bn + 1);
-            const float2 nf = __ffma2_rn(fm, f2(-1.0f, -1.0f), f2(MAGIC, MAGIC));   // -f
-            const float2 a0 = __fadd2_rn(t0, nf), am = __fadd2_rn(tm, __fadd2_rn(nf, f2(1.0f, 1.0f))),
-                         ap = __fadd2_rn(tp, __fadd2_rn(nf, f2(-1.0f, -1.0f)));
-            const float2 nr = f2(c1.x - q0.x, c1.x - qn.x), ng = f2(c1.y - q0.y, c1.y - qn.y),
-                         nb = f2(c1.z - q0.z, c1.z - qn.z);   // minus the colour differences
-            const uint32_t s0 = __float_as_uint(q0.w), sn = __float_as_uint(qn.w);
-            const PairSigns dm = pair_signs(pair_weight(am.x), Am), d0 = pair_signs(pair_weight(a0.x), A0),
-                            dp = pair_signs(pair_weight(ap.x), Ap);
-            const PairSigns em = pair_signs(pair_weight(am.y), Bm), e0 = pair_signs(pair_weight(a0.y), B0),
-                            ep = pair_signs(pair_weight(ap.y), Bp);
-            const int nm0 = pair_mismatch(dm, Am.x, s0), n00 = pair_mismatch(d0, A0.x, s0), np0 = pair_mismatch(dp, Ap.x, s0);
-            const int nm1 = pair_mismatch(em, Bm.x, sn), n01 = pair_mismatch(e0, B0.x, sn), np1 = pair_mismatch(ep, Bp.x, sn);
-            const uint32_t ma = __vimax3_s16x2(__vimax3_s16x2(dm.yw, dm.xz, d0.yw), __vimax3_s16x2(d0.xz, dp.yw, dp.xz), em.yw);
-            const uint32_t mb = __vimax3_s16x2(__vimax3_s16x2(em.xz, e0.yw, e0.xz), ep.yw, ep.xz);
-            // a weight in [0, 1) has bits below 1.0f's; a negative one or a NaN has not
-            const uint32_t wa = __vimax3_u32(__float_as_uint(am.x), __float_as_uint(a0.x), __float_as_uint(ap.x));
-            const uint32_t wb = __vimax3_u32(__float_as_uint(am.y), __float_as_uint(a0.y), __float_as_uint(ap.y));
-            const bool alone = sign_unsure(__vmaxs2(ma, mb)) || max(wa, wb) >= 0x3f800000u;
-            float2 w = support_weight2<F>(nr, ng, nb, one);
-            w.y = qx.y <= qx1 ? w.y : 0.0f;   // an odd row's last pair has one sample
-            const float2 k1 = __fmul2_rn(w, f2(PM_K033_8, PM_K033_8));
-            const float2 x = __fmul2_rn(w, f2(0.21875f, 0.21875f));   // (w * 0.875f) * 0.25, exact scaling
-            float2 Cm = tap2<F>(Am.x, Bm.x, A0.x, B0.x, am, __ffma2_rn(am, f2(-1.0f, -1.0f), f2(1.0f, 1.0f)), nr, ng, nb, k1,
-                                x, nm0, nm1, one);
-            float2 C = tap2<F>(A0.x, B0.x, A0.y, B0.y, a0, __ffma2_rn(a0, f2(-1.0f, -1.0f), f2(1.0f, 1.0f)), nr, ng, nb, k1,
-                               x, n00, n01, one);
-            float2 Cp = tap2<F>(A0.y, B0.y, Ap.y, Bp.y, ap, __ffma2_rn(ap, f2(-1.0f, -1.0f), f2(1.0f, 1.0f)), nr, ng, nb, k1,
-                                x, np0, np1, one);
-            if (alone) {
-                const float4* __restrict__ row2 = V.row2p(iy);
-                const float4* __restrict__ g2 = V.row2(iy) + V.plane;
-                Cm = tap_alone2<F>(__fadd2_rn(p, f2(-1.0f, -1.0f)), V, row2, g2, nr, ng, nb, s0, sn, k1, x);
-                C = tap_alone2<F>(p, V, row2, g2, nr, ng, nb, s0, sn, k1, x);
-                Cp = tap_alone2<F>(__fadd2_rn(p, f2(1.0f, 1.0f)), V, row2, g2, nr, ng, nb, s0, sn, k1, x);
-                // a non-finite column reads NaN texels for all three taps: equal costs, nothing added
-                if (!fin(p.x)) w.x = Cm.x = C.x = Cp.x = 0.0f;
-                if (!fin(p.y)) w.y = Cm.y = C.y = Cp.y = 0.0f;
-            }
-            // the update of :394-402 without a branch (KltSums)
-            const float2 curv = __ffma2_rn(C, f2(-2.0f, -2.0f), __fadd2_rn(Cp, Cm));   // 2 C is exact
-            const float2 wt = f2(curv.x > 0.0f ? w.x : 0.0f, curv.y > 0.0f ? w.y : 0.0f);
-            const float2 t = __fmul2_rn(wt, __ffma2_rn(Cp, f2(-1.0f, -1.0f), Cm)), sc = __fmul2_rn(wt, curv);
-            const float2 qy2 = f2(qy, qy);
-            A.J0 = accum2<F>(A.J0, t, qx);
-            A.J1 = accum2<F>(A.J1, t, qy2);
-            A.J2 = (A.J2 + t.x) + t.y;
-            A.h00 = accum2<F>(A.h00, sc, __fmul2_rn(qx, qx));
-            A.h01 = accum2<F>(A.h01, sc, __fmul2_rn(qx, qy2));
-            A.h02 = accum2<F>(A.h02, sc, qx);
-            A.h11 = accum2<F>(A.h11, sc, f2(qy * qy, qy * qy));
-            A.h12 = accum2<F>(A.h12, sc, qy2);
-            A.h22 = (A.h22 + sc.x) + sc.y;
-        }
+        const float4* __restrict__ row2 = V.row2p(iy);
+        const float4* __restrict__ g2 = V.row2(iy) + V.plane;
+        const float pa = match<F>(s, qx0, byq), pb = match<F>(s, qx1, byq);
+        const float plo = fminf(pa, pb), phi = fmaxf(pa, pb);
+        const bool even = pa >= 1.0f && pb >= 1.0f && phi < 4194304.0f &&
+                          ((__float_as_uint(phi + 1.5f) ^ __float_as_uint(plo)) < 0x00800000u);
+        const unsigned lanes = __activemask();
+        if (!__all_sync(lanes, even)) klt_row<F, false, false>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
+        // from column 256 on the weight is a multiple of 2^-15 and no sign is unsure
+        else if (__all_sync(lanes, plo >= 256.0f)) klt_row<F, true, true>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
+        else klt_row<F, true, false>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
     }
     const float3 d = lusolve(A.h00, A.h01, A.h02, A.h11, A.h12, A.h22, make_float3(A.J0 * 0.5f, A.J1 * 0.5f, A.J2 * 0.5f));
     return f4(s.x - d.x, s.y - d.y, s.z - d.z, s.w - 1e5f);
