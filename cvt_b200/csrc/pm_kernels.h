@@ -37,6 +37,7 @@ struct PropParams {
     float4* tmp_self;               // per-pixel state between the three propagate kernels
     float4* tmp_nb;
     int dual;                       // the window-loop kernels run as two variants (pm_window.cuh)
+    int owners;                     // pixels per warp row of the propagate kernels (set by the launchers)
 };
 
 // Batched launches over many pairs (pm_disparity_map_batch_device run in lockstep): a job is
@@ -65,7 +66,7 @@ void prop_tile_shape(int* w, int* h);
 // false for any other width
 bool prop_batch_tile_shape(int tile_w, int* w, int* h);
 // pairs per batched propagate launch: their arguments are one kernel parameter block
-// (128 x 184 bytes, within the 32,764 bytes a launch may pass)
+// (128 x 192 bytes, within the 32,764 bytes a launch may pass)
 constexpr int PROP_GROUP = 128;
 struct PropGroup {
     PropParams p[PROP_GROUP];

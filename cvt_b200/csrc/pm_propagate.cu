@@ -14,20 +14,17 @@
 #include <stdint.h>
 
 #include "pm_kernels.h"
+#include "pm_warp.cuh"
 
 namespace pm {
 
 namespace {
 
-// block shape: PM_PROP_BX consecutive pixels of a row (a warp is 32 of them, or two rows of 16
-// when PM_PROP_BX = 16), PM_PROP_BY rows per block
-#ifndef PM_PROP_BX
-#define PM_PROP_BX 32
-#endif
+// block shape of the single-pair kernels: PROP_BX consecutive threads, one warp, along a row, PM_PROP_BY rows
 #ifndef PM_PROP_BY
 #define PM_PROP_BY 4
 #endif
-constexpr int PROP_BX = PM_PROP_BX, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
+constexpr int PROP_BX = 32, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
 // Resident threads per SM asked of the register allocator for each kernel (640 = 96 registers, no
 // spills).  The window loops issue 88-92% of the cycles, so more threads give nothing: 1280x720,
 // r = 10, 3 iterations, ms (chain / Gauss-Newton): 512 threads 75.5 / 89.1, 640 69.2 / 88.9,
@@ -89,87 +86,112 @@ __device__ __forceinline__ bool known_outcome(float4 nb, float4 self, float thet
            __float_as_uint(nb.z) == __float_as_uint(self.z) && !(1.0f + theta * sd_self <= self.w + theta * sd_self);
 }
 
+// one warp's share of the shared memory of the window loops, and the calling lane (the block's warps are 32
+// consecutive threads, whatever its shape)
+__device__ __forceinline__ WarpScratch& warp_scratch(WarpScratch* ws, int& lane)
+{
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    lane = tid & 31;
+    return ws[tid >> 5];
+}
+
+// the window cost of the pixels of a warp whose lanes set `need` (all lanes call)
+template <bool F, bool COUNT, bool GEN, bool ROW>
+__device__ __forceinline__ float eval_pixels(const ViewData& V, WarpScratch* ws, bool need, int px, int py, float4 s,
+                                             float mincost, Counters& cnt)
+{
+    if (GEN) return need ? patch_eval_general<F, COUNT>(V, px, py, s, mincost, cnt) : 0.0f;
+    int lane;
+    WarpScratch& S = warp_scratch(ws, lane);
+    return patch_eval_warp<F, ROW>(V, S, lane, need, px, py, s, mincost);
+}
+
 // pmhstereo_propagate_view (:927-1028): candidates k = 0 (the current plane, re-evaluated,
 // :939-940), 1 smooth (:968-976), 2-5 random neighbours with offsets drawn x first, in
 // [-4, 5] (:982-991), 6 a random plane (:996-1002), 7-8 cross-view planes (:1007-1016),
 // 9 the randomized refinement (:1021-1028).  One loop, so that the window evaluation has a
-// single call site.
+// single call site, which the lanes of a warp reach together (eval_pixels).  A block covers
+// P.owners x BY pixels: the lanes threadIdx.x < P.owners own one each.
 template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
-__device__ __forceinline__ void chain_tile(const PropParams& P, int bx, int by, Counters& cnt)
+__device__ __forceinline__ void chain_tile(const PropParams& P, WarpScratch* ws, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
-    const int px = bx * BX + threadIdx.x, py = by * BY + threadIdx.y;
-    if (px < V.W && py < V.H) {
-        const int W = V.W;
-        const size_t idx = (size_t)py * W + px;
-        const float cx = (float)px, cy = (float)py;
-        const int lr = P.lr;
-        const float theta = P.theta, dmax = P.dmax;
-        float4 smooth = P.smooth[idx];
+    const int px = bx * P.owners + threadIdx.x, py = by * BY + threadIdx.y;
+    const bool own = threadIdx.x < P.owners && px < V.W && py < V.H;
+    if (GEN && !own) return;
+    const int W = V.W;
+    const size_t idx = (size_t)py * W + px;
+    const float cx = (float)px, cy = (float)py;
+    const int lr = P.lr;
+    const float theta = P.theta, dmax = P.dmax;
+    float4 smooth = f4(0.0f, 0.0f, 0.0f, 0.0f), self = smooth;
+    // cross-view candidates of this pixel; the entry is emptied for the next writer
+    int nview = 0;
+    unsigned long long vsrc = ~0ULL;
+    if (own) {
+        smooth = P.smooth[idx];
         smooth.w = clampf(smooth.w, 0.0f, 1.0f) * dmax;   // :927-928
-        float4 self = P.old[idx];
-
-        // cross-view candidates of this pixel; the entry is emptied for the next writer
-        int nview = 0;
-        unsigned long long vsrc = ~0ULL;
+        self = P.old[idx];
         if (P.vin_count) {
             nview = min(P.vin_count[idx], 2);
             vsrc = P.vin_src[idx];
             P.vin_count[idx] = 0;
             P.vin_src[idx] = ~0ULL;
         }
-
-        Rng rng;
-        // RNG_init(&rng, lin, ((1*1 - 1) + NUMRNDTRIES) * 3 + 2 * NUMRNDSAMPLE) (:942) expands to
-        // (lin) * ((1*1 - 1) + 2) * 3 + 2 * 4 = 6 * lin + 8
-        rng.init_skip((py * W + px + P.iter) * 6 + 8);
-
-        float sd_self = 0.0f;   // smoothing distance of `self` (smoothDistance does not read the cost)
-        for (int k = 0; k < 10; k++) {
-            float4 nb;
-            if (k == 0) {
-                nb = self;
-            } else if (k == 1) {
-                nb = from_disparity_normal(cx, cy, smooth.w * (lr ? -1.0f : 1.0f),
-                                           normalize3(make_float3(smooth.x, smooth.y, smooth.z)));
-                if (!lr) nb = viewprop(nb);
-            } else if (k <= 5) {
-                const int ox = (int)((rng.next() - 0.5f) * 2.0f * 5.0f + 0.5f);
-                const int oy = (int)((rng.next() - 0.5f) * 2.0f * 5.0f + 0.5f);
-                nb = P.old[(size_t)min(max(py + oy, 0), V.H - 1) * W + min(max(px + ox, 0), W - 1)];
-            } else if (k == 6) {
-                nb = nd_state_init(rng, cx, cy, lr, dmax);
-            } else if (k <= 8) {
-                if (k - 7 >= nview) continue;
-                nb = viewprop(P.vin_planes[(size_t)py * W + (k == 7 ? (unsigned int)vsrc : (unsigned int)(vsrc >> 32))]);
-            } else {
-                nb = nd_state_refine(rng, self, cx, cy, dmax, lr);
-            }
-            if (k == 0) {
-                self.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, 1e10f, cnt);
-                sd_self = smooth_dist1(self, smooth, cx, cy, dmax, lr);
-            } else {
-                if (known_outcome(nb, self, theta, sd_self)) continue;
-                const float sd = smooth_dist1(nb, smooth, cx, cy, dmax, lr);
-                // minimalCost (:873-877)
-                const float mincost = self.w + theta * sd_self - theta * sd;
-                nb.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, mincost, cnt);
-                if (nb.w + theta * sd <= self.w + theta * sd_self) {   // :976 etc.
-                    self = nb;
-                    sd_self = sd;
-                }
-            }
-        }
-        P.tmp_self[idx] = self;
     }
+
+    Rng rng;
+    // RNG_init(&rng, lin, ((1*1 - 1) + NUMRNDTRIES) * 3 + 2 * NUMRNDSAMPLE) (:942) expands to
+    // (lin) * ((1*1 - 1) + 2) * 3 + 2 * 4 = 6 * lin + 8
+    rng.init_skip((py * W + px + P.iter) * 6 + 8);
+
+    float sd_self = 0.0f;   // smoothing distance of `self` (smoothDistance does not read the cost)
+    for (int k = 0; k < 10; k++) {
+        float4 nb = self;
+        bool need = own;
+        if (k == 1) {
+            nb = from_disparity_normal(cx, cy, smooth.w * (lr ? -1.0f : 1.0f),
+                                       normalize3(make_float3(smooth.x, smooth.y, smooth.z)));
+            if (!lr) nb = viewprop(nb);
+        } else if (k >= 2 && k <= 5) {
+            const int ox = (int)((rng.next() - 0.5f) * 2.0f * 5.0f + 0.5f);
+            const int oy = (int)((rng.next() - 0.5f) * 2.0f * 5.0f + 0.5f);
+            if (own) nb = P.old[(size_t)min(max(py + oy, 0), V.H - 1) * W + min(max(px + ox, 0), W - 1)];
+        } else if (k == 6) {
+            nb = nd_state_init(rng, cx, cy, lr, dmax);
+        } else if (k == 7 || k == 8) {
+            need = k - 7 < nview;
+            if (need)
+                nb = viewprop(P.vin_planes[(size_t)py * W + (k == 7 ? (unsigned int)vsrc : (unsigned int)(vsrc >> 32))]);
+        } else if (k == 9) {
+            nb = nd_state_refine(rng, self, cx, cy, dmax, lr);
+        }
+        float sd = 0.0f, mincost = 1e10f;
+        if (k > 0) {
+            need = need && !known_outcome(nb, self, theta, sd_self);
+            sd = smooth_dist1(nb, smooth, cx, cy, dmax, lr);
+            // minimalCost (:873-877)
+            mincost = self.w + theta * sd_self - theta * sd;
+        }
+        nb.w = eval_pixels<F, COUNT, GEN, BX == 32>(V, ws, need, px, py, nb, mincost, cnt);
+        if (k == 0) {
+            self.w = nb.w;
+            sd_self = smooth_dist1(self, smooth, cx, cy, dmax, lr);
+        } else if (need && nb.w + theta * sd <= self.w + theta * sd_self) {   // :976 etc.
+            self = nb;
+            sd_self = sd;
+        }
+    }
+    if (own) P.tmp_self[idx] = self;
 }
 
 template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS, PM_CHAIN_BLOCKS) k_prop_chain(PropParams P)
 {
     if (variant_skips<GEN>(P.V, P.dual)) return;
+    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
     Counters cnt = {0, 0, 0, 0};
-    chain_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
+    chain_tile<F, COUNT, GEN>(P, ws, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
@@ -196,28 +218,50 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt(PropPa
     flush_counters<COUNT>(cnt, P.counters);
 }
 
+// the same with P.owners <= WARP_KLT pixels per warp (prop_owners)
+template <bool F>
+__global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt_warp(PropParams P)
+{
+    if (variant_skips<false>(P.V, P.dual)) return;
+    __shared__ WarpScratch ws[PROP_THREADS / 32];
+    const ViewData& V = P.V;
+    int lane;
+    WarpScratch& S = warp_scratch(ws, lane);
+    const int px = blockIdx.x * P.owners + threadIdx.x, py = blockIdx.y * PROP_BY + threadIdx.y;
+    if (py >= V.H) return;   // a warp is a row of the block
+    const bool own = threadIdx.x < P.owners && px < V.W;
+    const size_t idx = (size_t)py * V.W + px;
+    float4 nb = own ? P.tmp_self[idx] : f4(0.0f, 0.0f, 0.0f, 0.0f);
+    nb = klt2_steps_warp<F>(V, S, lane, P.owners, own, px, py, nb);
+    if (own) P.tmp_nb[idx] = nb;
+}
+
 // evaluation of the Gauss-Newton result (:1039-1052), view scatter (:1060-1067), output (:1070)
 template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
-__device__ __forceinline__ void final_tile(const PropParams& P, int bx, int by, Counters& cnt)
+__device__ __forceinline__ void final_tile(const PropParams& P, WarpScratch* ws, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
-    const int px = bx * BX + threadIdx.x, py = by * BY + threadIdx.y;
-    if (px < V.W && py < V.H) {
-        const int W = V.W;
-        const size_t idx = (size_t)py * W + px;
-        const float cx = (float)px, cy = (float)py;
-        const int lr = P.lr;
-        const float dmax = P.dmax, theta = P.theta;
-        float4 smooth = P.smooth[idx];
+    const int px = bx * P.owners + threadIdx.x, py = by * BY + threadIdx.y;
+    const bool own = threadIdx.x < P.owners && px < V.W && py < V.H;
+    if (GEN && !own) return;
+    const int W = V.W;
+    const size_t idx = (size_t)py * W + px;
+    const float cx = (float)px, cy = (float)py;
+    const int lr = P.lr;
+    const float dmax = P.dmax, theta = P.theta;
+    float4 smooth = f4(0.0f, 0.0f, 0.0f, 0.0f), self = smooth, nb = smooth;
+    if (own) {
+        smooth = P.smooth[idx];
         smooth.w = clampf(smooth.w, 0.0f, 1.0f) * dmax;
-        float4 self = P.tmp_self[idx];
-        float4 nb = P.tmp_nb[idx];
-        const float2 sd = smooth_distance(nb, self, smooth, cx, cy, dmax, lr);
-        if (!known_outcome(nb, self, theta, sd.y)) {
-            const float mincost = self.w + theta * sd.y - theta * sd.x;
-            nb.w = patch_eval<F, COUNT, GEN>(V, px, py, nb, mincost, cnt);
-            if (nb.w + theta * sd.x <= self.w + theta * sd.y) self = nb;
-        }
+        self = P.tmp_self[idx];
+        nb = P.tmp_nb[idx];
+    }
+    const float2 sd = smooth_distance(nb, self, smooth, cx, cy, dmax, lr);
+    const bool need = own && !known_outcome(nb, self, theta, sd.y);
+    const float mincost = self.w + theta * sd.y - theta * sd.x;
+    nb.w = eval_pixels<F, COUNT, GEN, BX == 32>(V, ws, need, px, py, nb, mincost, cnt);
+    if (own) {
+        if (need && nb.w + theta * sd.x <= self.w + theta * sd.y) self = nb;
 
         if (P.vout_count) {
             const float sidesign = lr ? -1.0f : 1.0f;
@@ -238,8 +282,9 @@ template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS) k_prop_final(PropParams P)
 {
     if (variant_skips<GEN>(P.V, P.dual)) return;
+    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
     Counters cnt = {0, 0, 0, 0};
-    final_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
+    final_tile<F, COUNT, GEN>(P, ws, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
@@ -253,6 +298,7 @@ template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_chain_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
+    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
     for (;;) {
         const int j = grab_job(next);
         if (j >= njobs) return;
@@ -260,7 +306,7 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
         const PropParams& P = G.p[job.x];
         if (variant_skips<GEN>(P.V, P.dual)) continue;
         Counters cnt = {0, 0, 0, 0};
-        chain_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
+        chain_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, ws, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
         flush_counters<COUNT>(cnt, P.counters);
     }
 }
@@ -285,6 +331,7 @@ template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_final_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
+    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
     for (;;) {
         const int j = grab_job(next);
         if (j >= njobs) return;
@@ -292,7 +339,7 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
         const PropParams& P = G.p[job.x];
         if (variant_skips<GEN>(P.V, P.dual)) continue;
         Counters cnt = {0, 0, 0, 0};
-        final_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
+        final_tile<F, COUNT, GEN, BX, PROP_THREADS / BX>(P, ws, (int)(job.y & 0xffffu), (int)(job.y >> 16), cnt);
         flush_counters<COUNT>(cnt, P.counters);
     }
 }
@@ -359,7 +406,10 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
 {
     if (J.njobs <= 0 || n < 1 || n > PROP_GROUP) return;
     static thread_local PropGroup tab;   // 23 KB: off the stack; copied into the launch
-    for (int i = 0; i < n; i++) tab.p[i] = group[i];
+    for (int i = 0; i < n; i++) {
+        tab.p[i] = group[i];
+        tab.p[i].owners = tile_w;
+    }
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
@@ -380,43 +430,67 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
     }
 }
 
-void launch_propagate(const PropParams& P, int fused, cudaStream_t st)
+// Pixels per warp of a single-pair pass over W x H pixels: a thread per pixel (32) unless the image is so
+// small that its warps, one thread's serial windows each, leave the chip idle.  Measured, ms a
+// call (two views, 5 iterations) with 32 / 16 / 8 / 4 / 2 / 1 pixels: 64x48, r = 5: - / - / 4.10 / 3.42 /
+// 3.00 / 3.44; 80x60, r = 7: - / 9.17 / 5.81 / 4.80 / 4.41 / 5.20; 120x90, r = 10: 13.8 / 18.1 / 12.1 / 10.2 /
+// 10.5 / -; 120x90, r = 3: 3.60 / 4.18 / 3.48 / 3.37 / 3.86 / -; 160x120, r = 7: 8.2 / 11.7 / 9.7 / 9.5;
+// 220x160, r = 5: 6.7 / 9.2 / 9.7.  Shared windows take 1.6 times the instructions, so they win only while
+// about 3000 warps (20 per SM) hold the image with at most 4 pixels each.
+int prop_owners(int W, int H)
+{
+    constexpr long long WARPS = 2960;
+    const long long n = (long long)W * H;
+    return n <= 2 * WARPS ? 2 : n <= 4 * WARPS ? 4 : 32;
+}
+
+namespace {
+
+template <bool F>
+void launch_pass(const PropParams& Q, cudaStream_t st)
 {
     const dim3 b(PROP_BX, PROP_BY);
-    const dim3 g = grid2d(P.V.W, P.V.H, b);
-    const bool count = P.counters != nullptr;
-#define PM_PROP_LAUNCH(FF, CC, KK, PP)                  \
-    do {                                                \
-        k_prop_chain<FF, CC, KK><<<g, b, 0, st>>>(PP);  \
-        k_prop_klt<FF, CC, KK><<<g, b, 0, st>>>(PP);    \
-        k_prop_final<FF, CC, KK><<<g, b, 0, st>>>(PP);  \
-    } while (0)
+    const dim3 g = grid2d(Q.V.W, Q.V.H, dim3(Q.owners, PROP_BY)), gg = grid2d(Q.V.W, Q.V.H, b);
+    PropParams G = Q;
+    G.owners = PROP_BX;
+    // both variants; the one that does not apply returns at once (pm_window.cuh).  Each kernel of the
+    // pass finishes before the next starts, for either variant.
+    k_prop_chain<F, false, false><<<g, b, 0, st>>>(Q);
+    k_prop_chain<F, false, true><<<gg, b, 0, st>>>(G);
+    if (Q.owners <= WARP_KLT) k_prop_klt_warp<F><<<g, b, 0, st>>>(Q);
+    else k_prop_klt<F, false, false><<<gg, b, 0, st>>>(G);
+    k_prop_klt<F, false, true><<<gg, b, 0, st>>>(G);
+    k_prop_final<F, false, false><<<g, b, 0, st>>>(Q);
+    k_prop_final<F, false, true><<<gg, b, 0, st>>>(G);
+}
+
+// counted passes: the general variant alone, which counts
+template <bool F>
+void launch_pass_counted(const PropParams& Q, cudaStream_t st)
+{
+    const dim3 b(PROP_BX, PROP_BY);
+    const dim3 g = grid2d(Q.V.W, Q.V.H, b);
+    k_prop_chain<F, true, true><<<g, b, 0, st>>>(Q);
+    k_prop_klt<F, true, true><<<g, b, 0, st>>>(Q);
+    k_prop_final<F, true, true><<<g, b, 0, st>>>(Q);
+}
+
+}  // namespace
+
+void launch_propagate(const PropParams& P, int fused, cudaStream_t st)
+{
     PropParams Q = P;
-    if (!count) {
-        // both variants; the one that does not apply returns at once (pm_window.cuh).  Each
-        // kernel of the pass finishes before the next starts, for either variant.
-        Q.dual = 1;
-        if (fused) {
-            k_prop_chain<true, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_chain<true, false, true><<<g, b, 0, st>>>(Q);
-            k_prop_klt<true, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_klt<true, false, true><<<g, b, 0, st>>>(Q);
-            k_prop_final<true, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_final<true, false, true><<<g, b, 0, st>>>(Q);
-        } else {
-            k_prop_chain<false, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_chain<false, false, true><<<g, b, 0, st>>>(Q);
-            k_prop_klt<false, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_klt<false, false, true><<<g, b, 0, st>>>(Q);
-            k_prop_final<false, false, false><<<g, b, 0, st>>>(Q);
-            k_prop_final<false, false, true><<<g, b, 0, st>>>(Q);
-        }
-    } else {
+    if (P.counters) {
         Q.dual = 0;
-        if (fused) PM_PROP_LAUNCH(true, true, true, Q);
-        else PM_PROP_LAUNCH(false, true, true, Q);
+        Q.owners = PROP_BX;
+        if (fused) launch_pass_counted<true>(Q, st);
+        else launch_pass_counted<false>(Q, st);
+    } else {
+        Q.dual = 1;
+        Q.owners = prop_owners(P.V.W, P.V.H);
+        if (fused) launch_pass<true>(Q, st);
+        else launch_pass<false>(Q, st);
     }
-#undef PM_PROP_LAUNCH
 }
 
 }  // namespace pm

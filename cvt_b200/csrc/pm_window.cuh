@@ -546,74 +546,74 @@ __device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, uintptr
     return m;
 }
 
-// patch_eval_census (:661-736) over pair records.
-//
-// The census only grows (every term is >= 0), so the source's exit test after each sample,
-// `census / bilw >= mincost` with a sample counted (:724), is decided by the census at the row's
-// end; it is tested there as census >= exit_threshold(mincost, bilw).
-//
-// p2x is monotone along a row, so its two ends decide, for the warp, whether samples can lie outside
-// the image or a column be non-finite.  From column 256 on a tap weight is a multiple of
-// 2^-15 and no sign is unsure.  Rows with a non-finite column and rows where some sign was
-// unsure run sample by sample with the signs from the gradients.
+// A row iy of patch_eval_pair, for the lanes that call it together.  p2x is monotone along a row, so its
+// two ends decide, for the warp, whether samples can lie outside the image or a column be
+// non-finite.  From column 256 on a tap weight is a multiple of 2^-15 and no sign is unsure.
+// Rows with a non-finite column and rows where some sign was unsure run sample by sample with the
+// signs from the gradients.
+template <bool F>
+__device__ __forceinline__ void eval_row_pixel(const ViewData& V, int iy, float4 s, float byq, float4 in, float qx0,
+                                               float qx1, float& census, float& wsum)
+{
+    const float fW = (float)V.W;
+    const float4* __restrict__ q1 = V.row1c(iy) + (int)qx0;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(V.row2p(iy)) - (uintptr_t)0x4B000000u * 16u;
+    const float pa = match<F>(s, qx0, byq), pb = match<F>(s, qx1, byq);
+    const float plo = fminf(pa, pb), phi = fmaxf(pa, pb);
+    const float census0 = census, wsum0 = wsum;
+    const bool in_image = pa >= 0.0f && pb >= 0.0f && phi < fW;
+    const bool sure = in_image && plo >= 256.0f;
+    const unsigned lanes = __activemask();
+    bool single = true;
+    if (__all_sync(lanes, sure)) {
+        eval_row<F, true, true>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW);
+        single = false;
+    } else if (__all_sync(lanes, in_image)) {
+        single = unsure(eval_row<F, true, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
+    } else if (__all_sync(lanes, fin(pa) && fin(pb))) {
+        if (!__any_sync(lanes, plo < fW && phi >= 0.0f)) return;
+        single = unsure(eval_row<F, false, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
+    }
+    if (!single) return;
+    census = census0;
+    wsum = wsum0;
+    const float4* __restrict__ g2 = V.row2(iy) + V.plane;
+    for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
+        const float p2x = match<F>(s, qx, byq);
+        if (p2x < 0 || p2x >= fW) continue;
+        const float4 q = __ldg(q1);
+        const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
+        float cost;
+        if (p2x == p2x) {
+            PairSigns d;
+            float a;
+            const float t = (p2x + 0.5f) - 0.5f;
+            cost = eval_sample_pair<F>(base, q, t, d, a);
+            cost = fmaf(0.21875f, (float)exact_mismatch<F>(g2 + (int)t, a, __float_as_uint(q.w)), cost);
+        } else {   // a NaN column reads the positive quiet NaN: full colour cost, positive signs
+            cost = fmaf(0.21875f, (float)sign_mismatch(__float_as_uint(q.w), 0u), PM_K033_8 * 3.0f);
+        }
+        census = F ? fmaf(w, cost, census) : census + w * cost;
+        wsum += w;
+    }
+}
+
+// patch_eval_census (:661-736) over pair records.  The census only grows (every term is >= 0), so the
+// source's exit test after each sample, `census / bilw >= mincost` with a sample counted (:724), is
+// decided by the census at the row's end; it is tested there as
+// census >= exit_threshold(mincost, bilw).
 template <bool F>
 __device__ __forceinline__ float patch_eval_pair(const ViewData& V, int px, int py, float4 s, float mincost)
 {
     const float cx = (float)px, cy = (float)py;
     if (!plane_usable(s, cx, cy, V.W)) return 1e5f;
-    const int W = V.W;
     const float4 in = __ldg(V.row1(py) + px);
     const float thr = exit_threshold(mincost, in.w);
     float wsum = 0.0f, census = 0.0f;
     const int r = V.r;
-    const int dy0 = max(-r, -py), dy1 = min(r, V.H - 1 - py);
-    const int dx0 = max(-r, -px), dx1 = min(r, W - 1 - px);
-    const float fW = (float)W;
-    const float qx0 = cx + (float)dx0, qx1 = cx + (float)dx1;
-    float qy = cy + (float)dy0;
-    for (int iy = py + dy0; iy <= py + dy1; iy++, qy += 1.0f) {
-        const float byq = s.y * qy;
-        const float4* __restrict__ q1 = V.row1c(iy) + px + dx0;
-        const uintptr_t base = reinterpret_cast<uintptr_t>(V.row2p(iy)) - (uintptr_t)0x4B000000u * 16u;
-        const float pa = match<F>(s, qx0, byq), pb = match<F>(s, qx1, byq);
-        const float plo = fminf(pa, pb), phi = fmaxf(pa, pb);
-        const float census0 = census, wsum0 = wsum;
-        const bool in_image = pa >= 0.0f && pb >= 0.0f && phi < fW;
-        const bool sure = in_image && plo >= 256.0f;
-        const unsigned lanes = __activemask();
-        bool single = true;
-        if (__all_sync(lanes, sure)) {
-            eval_row<F, true, true>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW);
-            single = false;
-        } else if (__all_sync(lanes, in_image)) {
-            single = unsure(eval_row<F, true, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
-        } else if (__all_sync(lanes, fin(pa) && fin(pb))) {
-            if (!__any_sync(lanes, plo < fW && phi >= 0.0f)) continue;
-            single = unsure(eval_row<F, false, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
-        }
-        if (single) {
-            census = census0;
-            wsum = wsum0;
-            const float4* __restrict__ g2 = V.row2(iy) + V.plane;
-            for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
-                const float p2x = match<F>(s, qx, byq);
-                if (p2x < 0 || p2x >= fW) continue;
-                const float4 q = __ldg(q1);
-                const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
-                float cost;
-                if (p2x == p2x) {
-                    PairSigns d;
-                    float a;
-                    const float t = (p2x + 0.5f) - 0.5f;
-                    cost = eval_sample_pair<F>(base, q, t, d, a);
-                    cost = fmaf(0.21875f, (float)exact_mismatch<F>(g2 + (int)t, a, __float_as_uint(q.w)), cost);
-                } else {   // a NaN column reads the positive quiet NaN: full colour cost, positive signs
-                    cost = fmaf(0.21875f, (float)sign_mismatch(__float_as_uint(q.w), 0u), PM_K033_8 * 3.0f);
-                }
-                census = F ? fmaf(w, cost, census) : census + w * cost;
-                wsum += w;
-            }
-        }
+    const float qx0 = (float)max(px - r, 0), qx1 = (float)min(px + r, V.W - 1);
+    for (int iy = max(py - r, 0); iy <= min(py + r, V.H - 1); iy++) {
+        eval_row_pixel<F>(V, iy, s, s.y * (float)iy, in, qx0, qx1, census, wsum);
         if (census >= thr && wsum > 0.0f) return 1.0f;
     }
     if (wsum <= 1.0f) return 1.1f;
@@ -662,8 +662,10 @@ __device__ __forceinline__ float tap_alone(float u, int W, const float4* __restr
     return tap_cost(k1, x, tap_ad<F>(pair_rgb(R.x), pair_rgb(R.y), a, 1.0f - a, nref), exact_mismatch<F>(g2 + c, a, sb1));
 }
 
-// A row of klt2_pair (row2, g2: column 0 of the pair and gradient rows).
-// EVEN: every p2x is at least 1 with p2x + 1.5 in the same binade, below 2^22.  p2x is then a
+// The terms of a window sample of a Gauss-Newton step (:350-402): t = w (Cxm - Cxp), twice the factor of
+// J's sums, and sc = w curv, the factor of H's; both +-0 for a rejected sample.  q: compact texel,
+// c1: centre colour, p2x: matched column; row2, g2: column 0 of the pair and gradient rows.
+// EVEN: p2x is at least 1 with p2x + 1.5 in the same binade, below 2^22.  p2x is then a
 // multiple of its ulp <= 0.5, the +-1 and +-0.5 of the source are exact, and the taps at t - 1, t,
 // t + 1 share the weight p2x - floor(p2x).  Otherwise each tap's coordinate is formed as the source
 // forms it; mostly the floors are still f - 1, f, f + 1 and only the weights differ in the last bit, and the
@@ -673,58 +675,66 @@ __device__ __forceinline__ float tap_alone(float u, int W, const float4* __restr
 // source's clamp gives.  Where a weight is out of range (floors that do not chain, a non-finite column) or,
 // not SURE, a sign unsure, each tap is read on its own.
 template <bool F, bool EVEN, bool SURE>
-__device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restrict__ row2, const float4* __restrict__ g2,
-                                        const float4* __restrict__ q1, float4 c1, float4 s, float byq, float qx0, float qx1,
-                                        float qy)
+__device__ __forceinline__ void klt_terms(int W, const float4* __restrict__ row2, const float4* __restrict__ g2, float4 q,
+                                          float4 c1, float p2x, float& t, float& sc)
 {
     const float MAGIC = EVEN ? 8388608.0f : 12582912.0f;   // MAGIC + t rounded down: MAGIC + floor(t), t >= 0 or |t| < 2^22
     // column c of the row is at base + 16 * (bits of the float MAGIC + c)
     const uintptr_t base = reinterpret_cast<uintptr_t>(row2) - (uintptr_t)(EVEN ? 0x4B000000u : 0x4B400000u) * 16u;
     const float first = MAGIC - 3.0f, last = MAGIC + (float)(W + 1);
+    const float t0 = EVEN ? p2x : (p2x + 0.5f) - 0.5f;
+    const float fm = __fadd_rd(t0, MAGIC);
+    const float fc = EVEN ? fminf(fm, last) : fminf(fmaxf(fm, first), last);
+    const uint4* b = reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fc) * 16u);
+    const PairRec Rm = __ldg(b - 1), R0 = __ldg(b), Rp = __ldg(b + 1);
+    const float f = fm - MAGIC;
+    const float a0 = t0 - f;
+    float am = a0, ap = a0;
+    if (!EVEN) {
+        am = (((p2x + -1.0f) + 0.5f) - 0.5f) - (f - 1.0f);
+        ap = (((p2x + 1.0f) + 0.5f) - 0.5f) - (f + 1.0f);
+    }
+    const uint32_t A0 = pair_weight(a0), Am = EVEN ? A0 : pair_weight(am), Ap = EVEN ? A0 : pair_weight(ap);
+    const uint32_t sb1 = __float_as_uint(q.w);
+    const PairSigns dm = pair_signs(Am, Rm), d0 = pair_signs(A0, R0), dp = pair_signs(Ap, Rp);
+    const float3 nref = make_float3(c1.x - q.x, c1.y - q.y, c1.z - q.z);   // minus the colour difference
+    float w1 = support_weight<F>(nref.x, nref.y, nref.z);
+    const float k1 = w1 * PM_K033_8, x = w1 * 0.21875f;   // (w1 * 0.875f) * 0.25, exact scaling
+    const float b0 = 1.0f - a0, bm = EVEN ? b0 : 1.0f - am, bp = EVEN ? b0 : 1.0f - ap;
+    const float3 tA = pair_rgb(Rm.x), tB = pair_rgb(R0.x);
+    float Cm = tap_cost(k1, x, tap_ad<F>(tA, tB, am, bm, nref), pair_mismatch(dm, sb1));
+    const float3 tC = pair_rgb(R0.y);
+    float C = tap_cost(k1, x, tap_ad<F>(tB, tC, a0, b0, nref), pair_mismatch(d0, sb1));
+    const float3 tD = pair_rgb(Rp.y);
+    float Cp = tap_cost(k1, x, tap_ad<F>(tC, tD, ap, bp, nref), pair_mismatch(dp, sb1));
+    bool alone = false;
+    if (!SURE) alone = unsure(unsure_max(unsure_max(unsure_max(0u, dm), d0), dp));
+    // a weight in [0, 1) has bits below 1.0f's; a negative one or a NaN has not
+    if (!EVEN) alone |= max(max(__float_as_uint(am), __float_as_uint(a0)), __float_as_uint(ap)) >= 0x3f800000u;
+    if (alone) {
+        Cm = tap_alone<F>(p2x + -1.0f, W, row2, g2, nref, sb1, k1, x);
+        C = tap_alone<F>(p2x, W, row2, g2, nref, sb1, k1, x);
+        Cp = tap_alone<F>(p2x + 1.0f, W, row2, g2, nref, sb1, k1, x);
+        // a non-finite column reads NaN texels for all three taps: equal costs, nothing added
+        if (!fin(p2x)) w1 = Cm = C = Cp = 0.0f;
+    }
+    // the update of :394-402 without a branch
+    const float curv = fmaf(-2.0f, C, Cp + Cm);   // 2 C is exact
+    const float wt = curv > 0.0f ? w1 : 0.0f;
+    t = wt * (Cm - Cp);
+    sc = wt * curv;
+}
+
+// a row of klt2_pair
+template <bool F, bool EVEN, bool SURE>
+__device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restrict__ row2, const float4* __restrict__ g2,
+                                        const float4* __restrict__ q1, float4 c1, float4 s, float byq, float qx0, float qx1,
+                                        float qy)
+{
     const float yy = qy * qy;
     for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
-        const float4 q = __ldg(q1);
-        const float p2x = match<F>(s, qx, byq);
-        const float t0 = EVEN ? p2x : (p2x + 0.5f) - 0.5f;
-        const float fm = __fadd_rd(t0, MAGIC);
-        const float fc = EVEN ? fminf(fm, last) : fminf(fmaxf(fm, first), last);
-        const uint4* b = reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fc) * 16u);
-        const PairRec Rm = __ldg(b - 1), R0 = __ldg(b), Rp = __ldg(b + 1);
-        const float f = fm - MAGIC;
-        const float a0 = t0 - f;
-        float am = a0, ap = a0;
-        if (!EVEN) {
-            am = (((p2x + -1.0f) + 0.5f) - 0.5f) - (f - 1.0f);
-            ap = (((p2x + 1.0f) + 0.5f) - 0.5f) - (f + 1.0f);
-        }
-        const uint32_t A0 = pair_weight(a0), Am = EVEN ? A0 : pair_weight(am), Ap = EVEN ? A0 : pair_weight(ap);
-        const uint32_t sb1 = __float_as_uint(q.w);
-        const PairSigns dm = pair_signs(Am, Rm), d0 = pair_signs(A0, R0), dp = pair_signs(Ap, Rp);
-        const float3 nref = make_float3(c1.x - q.x, c1.y - q.y, c1.z - q.z);   // minus the colour difference
-        float w1 = support_weight<F>(nref.x, nref.y, nref.z);
-        const float k1 = w1 * PM_K033_8, x = w1 * 0.21875f;   // (w1 * 0.875f) * 0.25, exact scaling
-        const float b0 = 1.0f - a0, bm = EVEN ? b0 : 1.0f - am, bp = EVEN ? b0 : 1.0f - ap;
-        const float3 tA = pair_rgb(Rm.x), tB = pair_rgb(R0.x);
-        float Cm = tap_cost(k1, x, tap_ad<F>(tA, tB, am, bm, nref), pair_mismatch(dm, sb1));
-        const float3 tC = pair_rgb(R0.y);
-        float C = tap_cost(k1, x, tap_ad<F>(tB, tC, a0, b0, nref), pair_mismatch(d0, sb1));
-        const float3 tD = pair_rgb(Rp.y);
-        float Cp = tap_cost(k1, x, tap_ad<F>(tC, tD, ap, bp, nref), pair_mismatch(dp, sb1));
-        bool alone = false;
-        if (!SURE) alone = unsure(unsure_max(unsure_max(unsure_max(0u, dm), d0), dp));
-        // a weight in [0, 1) has bits below 1.0f's; a negative one or a NaN has not
-        if (!EVEN) alone |= max(max(__float_as_uint(am), __float_as_uint(a0)), __float_as_uint(ap)) >= 0x3f800000u;
-        if (alone) {
-            Cm = tap_alone<F>(p2x + -1.0f, W, row2, g2, nref, sb1, k1, x);
-            C = tap_alone<F>(p2x, W, row2, g2, nref, sb1, k1, x);
-            Cp = tap_alone<F>(p2x + 1.0f, W, row2, g2, nref, sb1, k1, x);
-            // a non-finite column reads NaN texels for all three taps: equal costs, nothing added
-            if (!fin(p2x)) w1 = Cm = C = Cp = 0.0f;
-        }
-        // the update of :394-402 without a branch (KltSums)
-        const float curv = fmaf(-2.0f, C, Cp + Cm);   // 2 C is exact
-        const float wt = curv > 0.0f ? w1 : 0.0f;
-        const float t = wt * (Cm - Cp), sc = wt * curv;
+        float t, sc;
+        klt_terms<F, EVEN, SURE>(W, row2, g2, __ldg(q1), c1, match<F>(s, qx, byq), t, sc);
         if (F) {
             A.J0 = fmaf(t, qx, A.J0);
             A.J1 = fmaf(t, qy, A.J1);

@@ -260,6 +260,24 @@ def test_pair_plane_loops_match_oracle(D, orc, W, H, r, fused):
     assert bits_equal(host(D.klt(dP, dL, dR, dgL, dgR, r, fused)), orc.klt(P, bwL, bwR, gL, gR, r, fused=fused)).all()
 
 
+@pytest.mark.parametrize("fused", [0, 1])
+@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 5), (148, 80, 3), (149, 80, 4), (33, 400, 1)])
+def test_propagate_over_pair_planes_matches_oracle(D, orc, W, H, r, fused):
+    """One propagate pass from the planes of pair_planes: two, four and 32 pixels per warp (the bounds of
+    prop_owners among the sizes), windows of several passes over the shared memory, shared and single rows
+    in one window."""
+    rng = np.random.default_rng(7 * W + r)
+    L = rng.integers(0, 256, (H, W, 4), dtype=np.uint8)
+    R = np.clip(np.roll(L, -2, 1).astype(int) + rng.integers(-9, 10, L.shape), 0, 255).astype(np.uint8)
+    bwL, gL, _ = orc.prep(L, r, fused=fused)
+    bwR, gR, _ = orc.prep(R, r, fused=fused)
+    P = pair_planes(rng, W, H, gR)
+    sm = np.zeros((H, W, 4), np.float32)
+    want = orc.propagate(P, bwL, bwR, gL, gR, sm, 0.3, r, 16.0, 1, 2, fused=fused)[0]
+    got = D.propagate(*(dev(D.t, a) for a in (P, bwL, bwR, gL, gR, sm)), 0.3, r, 16.0, 1, 2, fused=fused)
+    assert bits_equal(host(got), want).all()
+
+
 def test_propagate_view_exchange_matches_oracle(D, orc):
     """Left propagate scatters into the view buffer, right propagate consumes it."""
     from cvt_b200 import scene
