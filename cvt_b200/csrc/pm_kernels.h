@@ -109,6 +109,8 @@ void launch_init(float4* out, const ViewData& V, float dmax, int lr, const float
 void launch_cost(float* cost, const float4* planes, const ViewData& V, float mincost, int fused, cudaStream_t st);
 void launch_klt(float4* out, const float4* planes, const ViewData& V, int fused, cudaStream_t st);
 void launch_propagate(const PropParams& P, int fused, cudaStream_t st);
+// pixels per warp of a window pass over one W x H image (pm_propagate.cu)
+int prop_owners(int W, int H);
 // launches per window-loop kernel (init, cost, klt, each of the three propagate kernels):
 // uncounted runs launch both variants (pm_window.cuh)
 inline int window_kernel_launches(int fused, bool counting)

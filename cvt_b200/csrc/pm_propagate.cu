@@ -88,7 +88,7 @@ __device__ __forceinline__ bool known_outcome(float4 nb, float4 self, float thet
 
 // one warp's share of the shared memory of the window loops, and the calling lane (the block's warps are 32
 // consecutive threads, whatever its shape)
-__device__ __forceinline__ WarpScratch& warp_scratch(WarpScratch* ws, int& lane)
+__device__ __forceinline__ WarpScratch<>& warp_scratch(WarpScratch<>* ws, int& lane)
 {
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     lane = tid & 31;
@@ -97,12 +97,12 @@ __device__ __forceinline__ WarpScratch& warp_scratch(WarpScratch* ws, int& lane)
 
 // the window cost of the pixels of a warp whose lanes set `need` (all lanes call)
 template <bool F, bool COUNT, bool GEN, bool ROW>
-__device__ __forceinline__ float eval_pixels(const ViewData& V, WarpScratch* ws, bool need, int px, int py, float4 s,
+__device__ __forceinline__ float eval_pixels(const ViewData& V, WarpScratch<>* ws, bool need, int px, int py, float4 s,
                                              float mincost, Counters& cnt)
 {
     if (GEN) return need ? patch_eval_general<F, COUNT>(V, px, py, s, mincost, cnt) : 0.0f;
     int lane;
-    WarpScratch& S = warp_scratch(ws, lane);
+    WarpScratch<>& S = warp_scratch(ws, lane);
     return patch_eval_warp<F, ROW>(V, S, lane, need, px, py, s, mincost);
 }
 
@@ -113,7 +113,7 @@ __device__ __forceinline__ float eval_pixels(const ViewData& V, WarpScratch* ws,
 // single call site, which the lanes of a warp reach together (eval_pixels).  A block covers
 // P.owners x BY pixels: the lanes threadIdx.x < P.owners own one each.
 template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
-__device__ __forceinline__ void chain_tile(const PropParams& P, WarpScratch* ws, int bx, int by, Counters& cnt)
+__device__ __forceinline__ void chain_tile(const PropParams& P, WarpScratch<>* ws, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
     const int px = bx * P.owners + threadIdx.x, py = by * BY + threadIdx.y;
@@ -189,7 +189,7 @@ template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS, PM_CHAIN_BLOCKS) k_prop_chain(PropParams P)
 {
     if (variant_skips<GEN>(P.V, P.dual)) return;
-    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
+    __shared__ WarpScratch<> ws[GEN ? 1 : PROP_THREADS / 32];
     Counters cnt = {0, 0, 0, 0};
     chain_tile<F, COUNT, GEN>(P, ws, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
@@ -223,22 +223,22 @@ template <bool F>
 __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt_warp(PropParams P)
 {
     if (variant_skips<false>(P.V, P.dual)) return;
-    __shared__ WarpScratch ws[PROP_THREADS / 32];
+    __shared__ WarpScratch<> ws[PROP_THREADS / 32];
     const ViewData& V = P.V;
     int lane;
-    WarpScratch& S = warp_scratch(ws, lane);
+    WarpScratch<>& S = warp_scratch(ws, lane);
     const int px = blockIdx.x * P.owners + threadIdx.x, py = blockIdx.y * PROP_BY + threadIdx.y;
     if (py >= V.H) return;   // a warp is a row of the block
     const bool own = threadIdx.x < P.owners && px < V.W;
     const size_t idx = (size_t)py * V.W + px;
     float4 nb = own ? P.tmp_self[idx] : f4(0.0f, 0.0f, 0.0f, 0.0f);
-    nb = klt2_steps_warp<F>(V, S, lane, P.owners, own, px, py, nb);
+    nb = klt2_steps_warp<F>(V, S, lane, P.owners, 6, own, px, py, nb);
     if (own) P.tmp_nb[idx] = nb;
 }
 
 // evaluation of the Gauss-Newton result (:1039-1052), view scatter (:1060-1067), output (:1070)
 template <bool F, bool COUNT, bool GEN, int BX = PROP_BX, int BY = PROP_BY>
-__device__ __forceinline__ void final_tile(const PropParams& P, WarpScratch* ws, int bx, int by, Counters& cnt)
+__device__ __forceinline__ void final_tile(const PropParams& P, WarpScratch<>* ws, int bx, int by, Counters& cnt)
 {
     const ViewData& V = P.V;
     const int px = bx * P.owners + threadIdx.x, py = by * BY + threadIdx.y;
@@ -282,7 +282,7 @@ template <bool F, bool COUNT, bool GEN>
 __global__ void __launch_bounds__(PROP_THREADS) k_prop_final(PropParams P)
 {
     if (variant_skips<GEN>(P.V, P.dual)) return;
-    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
+    __shared__ WarpScratch<> ws[GEN ? 1 : PROP_THREADS / 32];
     Counters cnt = {0, 0, 0, 0};
     final_tile<F, COUNT, GEN>(P, ws, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
@@ -298,7 +298,7 @@ template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_chain_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
-    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
+    __shared__ WarpScratch<> ws[GEN ? 1 : PROP_THREADS / 32];
     for (;;) {
         const int j = grab_job(next);
         if (j >= njobs) return;
@@ -331,7 +331,7 @@ template <bool F, bool COUNT, bool GEN, int BX>
 __global__ void __launch_bounds__(PROP_THREADS, PM_BATCH_BLOCKS)
     k_prop_final_b(const __grid_constant__ PropGroup G, const uint2* __restrict__ jobs, int njobs, int* next)
 {
-    __shared__ WarpScratch ws[GEN ? 1 : PROP_THREADS / 32];
+    __shared__ WarpScratch<> ws[GEN ? 1 : PROP_THREADS / 32];
     for (;;) {
         const int j = grab_job(next);
         if (j >= njobs) return;

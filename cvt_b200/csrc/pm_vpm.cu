@@ -8,11 +8,15 @@
 // disparities), `iterations` passes of vpmstereo_iter_simple (a van der Corput candidate,
 // eight neighbour states, three Gauss-Newton steps), then |x' - x|.
 //
-// Texel layout.  The first image is read only at integral texels and only through its colour
-// and the signs of its gradient, so it is one float4 plane: (r, g, b, the four gradient sign
-// bits as bytes).  The second image is read bilinearly along rows: a colour plane
-// (r, g, b, a) and a gradient plane, rows of W float4.  Plane states ping-pong between two
-// W*H float4 fields.
+// Texel layout.  Both images have the texel planes of pm_window.cuh: of the first the compact plane
+// (colour and gradient signs) and the colour plane's w component (the window's weight sum) are
+// read, of the second the pair plane, and by the general loops its colour and gradient planes.
+// Plane states ping-pong between two W*H float4 fields.
+//
+// A pass is three kernels, as the main path's (candidates, Gauss-Newton steps, their evaluation), over the
+// pair-plane loops of pm_window.cuh / pm_warp.cuh.  The general loops below, one kernel per pass, count the
+// taps (pm_vpm_set_counting) and serve injected gradients that are not finite.  Measured at 640x480, r = 10,
+// 8 iterations: general loops 95.7 ms a call, the three kernels 56.7 (30.2 + 21.9 + 3.6).
 //
 // Arithmetic is the reference's FP32 sequence (the file is compiled with -fmad=false): every
 // result equals the restatement in oracle/pm_oracle.cpp bit for bit.  The one double in the
@@ -26,7 +30,8 @@
 #include <string>
 
 #include "../../include/cvtpm.h"
-#include "pm_window.cuh"
+#include "pm_kernels.h"
+#include "pm_warp.cuh"
 
 namespace pm {
 namespace vpm {
@@ -37,12 +42,7 @@ constexpr float WEIGHT = 8.0f;       // CENSUS_COLOR_WEIGHT (:30)
 // per SM (80 registers): 13% faster than the compiler's 100-register choice at 2 blocks
 constexpr int BX = 32, BY = 8;
 
-struct Views {
-    const float4* __restrict__ t1;   // first image: (r, g, b, gradient sign bytes)
-    const float4* __restrict__ c2;   // second image: colour
-    const float4* __restrict__ g2;   // second image: gradient
-    int W, H, r;
-};
+typedef ViewData Views;
 
 __device__ __forceinline__ float unorm8(uint32_t v) { return __fdiv_rn((float)v, 255.0f); }
 
@@ -65,7 +65,7 @@ __device__ __forceinline__ float weight(float4 t, float4 ctr)
 
 // (1 - a) T0 + a T1 per component, each product and the sum rounded once (SAMPLER_BILINEAR
 // with the vertical weight 0, as lerp_row)
-__device__ __forceinline__ float4 mix(float a, float4 T0, float4 T1)
+__device__ __forceinline__ float4 mix4(float a, float4 T0, float4 T1)
 {
     const float b = 1.0f - a;
     return f4(__fadd_rn(__fmul_rn(b, T0.x), __fmul_rn(a, T1.x)), __fadd_rn(__fmul_rn(b, T0.y), __fmul_rn(a, T1.y)),
@@ -86,9 +86,9 @@ __device__ __forceinline__ void sample2(const Views& V, int row, float u, float4
     fl = fminf(fmaxf(fl, -1.0f), (float)V.W);
     const int i0 = (int)fl;
     const int j0 = min(max(i0, 0), V.W - 1), j1 = min(max(i0 + 1, 0), V.W - 1);
-    const size_t o = (size_t)row * V.W;
-    c = mix(a, __ldg(V.c2 + o + j0), __ldg(V.c2 + o + j1));
-    g = mix(a, __ldg(V.g2 + o + j0), __ldg(V.g2 + o + j1));
+    const float4 *c2 = V.row2(row), *g2 = c2 + V.plane;
+    c = mix4(a, __ldg(c2 + j0), __ldg(c2 + j1));
+    g = mix4(a, __ldg(g2 + j0), __ldg(g2 + j1));
 }
 
 // patch_eval_census (:200-258).  Taps outside the image or mapped outside the second image
@@ -99,14 +99,14 @@ __device__ float eval(const Views& V, int px, int py, float3 s, unsigned long lo
     const float cx = (float)px, cy = (float)py;
     const float c2x = s.x * cx + s.y * cy + s.z;
     if (c2x < 0 || c2x >= (float)V.W) return 1.0f;
-    const float4 ctr = __ldg(V.t1 + (size_t)py * V.W + px);
+    const float4 ctr = __ldg(V.row1c(py) + px);
     float wsum = 0.0f, census = 0.0f;
     const int ylo = max(py - V.r, 0), yhi = min(py + V.r, V.H - 1);
     const int xlo = max(px - V.r, 0), xhi = min(px + V.r, V.W - 1);
     for (int iy = ylo; iy <= yhi; iy++) {
         const float qy = cy + (float)(iy - py) * 1.0f;
         const float ry = s.y * qy;
-        const float4* row1 = V.t1 + (size_t)iy * V.W;
+        const float4* row1 = V.row1c(iy);
         for (int ix = xlo; ix <= xhi; ix++) {
             const float qx = cx + (float)(ix - px) * 1.0f;
             const float p2x = (s.x * qx + ry) + s.z;
@@ -143,15 +143,14 @@ __device__ float3 klt(const Views& V, int px, int py, float3 s, unsigned long lo
     const float cx = (float)px, cy = (float)py;
     float J0 = 0.0f, J1 = 0.0f, J2 = 0.0f;
     float h00 = 0.0f, h01 = 0.0f, h02 = 0.0f, h11 = 0.0f, h12 = 0.0f, h22 = 0.0f;
-    const float4 ctr = __ldg(V.t1 + (size_t)py * V.W + px);
+    const float4 ctr = __ldg(V.row1c(py) + px);
     const int ylo = max(py - V.r, 0), yhi = min(py + V.r, V.H - 1);
     // the taps that reach the cost: inside the image and not in its first or last column (:151)
     const int xlo = max(px - V.r, 1), xhi = min(px + V.r, V.W - 2);
     for (int iy = ylo; iy <= yhi; iy++) {
         const float qy = cy + (float)(iy - py) * 1.0f;
         const float ry = s.y * qy;
-        const float4* row1 = V.t1 + (size_t)iy * V.W;
-        const size_t o = (size_t)iy * V.W;
+        const float4 *row1 = V.row1c(iy), *rc = V.row2(iy), *rg = rc + V.plane;
         for (int ix = xlo; ix <= xhi; ix++) {
             const float qx = cx + (float)(ix - px) * 1.0f;
             const float4 t = __ldg(row1 + ix);
@@ -173,13 +172,13 @@ __device__ float3 klt(const Views& V, int px, int py, float3 s, unsigned long lo
                 if ((int)fp == i0 + 1 && (int)fm == i0 - 1) {
                     const int jm = min(max(i0 - 1, 0), V.W - 1), j0 = min(max(i0, 0), V.W - 1);
                     const int j1 = min(max(i0 + 1, 0), V.W - 1), j2 = min(max(i0 + 2, 0), V.W - 1);
-                    const float4 cm = __ldg(V.c2 + o + jm), c0 = __ldg(V.c2 + o + j0);
-                    const float4 c1 = __ldg(V.c2 + o + j1), c2 = __ldg(V.c2 + o + j2);
-                    const float4 gm = __ldg(V.g2 + o + jm), g0 = __ldg(V.g2 + o + j0);
-                    const float4 g1 = __ldg(V.g2 + o + j1), g2 = __ldg(V.g2 + o + j2);
-                    C = klt_tap(k1, kd, t, sb1, mix(a0, c0, c1), mix(a0, g0, g1));
-                    Cxp = klt_tap(k1, kd, t, sb1, mix(ap, c1, c2), mix(ap, g1, g2));
-                    Cxm = klt_tap(k1, kd, t, sb1, mix(am, cm, c0), mix(am, gm, g0));
+                    const float4 cm = __ldg(rc + jm), c0 = __ldg(rc + j0);
+                    const float4 c1 = __ldg(rc + j1), c2 = __ldg(rc + j2);
+                    const float4 gm = __ldg(rg + jm), g0 = __ldg(rg + j0);
+                    const float4 g1 = __ldg(rg + j1), g2 = __ldg(rg + j2);
+                    C = klt_tap(k1, kd, t, sb1, mix4(a0, c0, c1), mix4(a0, g0, g1));
+                    Cxp = klt_tap(k1, kd, t, sb1, mix4(ap, c1, c2), mix4(ap, g1, g2));
+                    Cxm = klt_tap(k1, kd, t, sb1, mix4(am, cm, c0), mix4(am, gm, g0));
                     done = true;
                 }
             }
@@ -212,32 +211,44 @@ __device__ float3 klt(const Views& V, int px, int py, float3 s, unsigned long lo
 
 // Colour texels and gradients of one image (grad_gray_xydiag, gradxy.cl:60-97: central grey
 // differences with the zero border of CLK_ADDRESS_CLAMP, the diagonal channels repeating
-// them), or the caller's gradient image when gin is given.  Writes any of: the first-image
-// compact plane, the colour plane, the gradient plane.
-__global__ void k_prep(const uint8_t* __restrict__ img, size_t stride, int W, int H, const float4* __restrict__ gin,
-                       float4* __restrict__ compact, float4* __restrict__ colour, float4* __restrict__ grad)
+// them), or the caller's gradient image when gin is given.  Writes any of: the colour plane, with r >= 0
+// the window's weight sum in its w component, and the gradient plane.
+__global__ void k_prep(const uint8_t* __restrict__ img, size_t stride, int W, int H, int r, const float4* __restrict__ gin,
+                       float4* __restrict__ colour, float4* __restrict__ grad)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;
     auto px = [&](int xx, int yy) { return __ldg(reinterpret_cast<const uchar4*>(img + (size_t)yy * stride) + xx); };
+    auto rgb = [&](int xx, int yy) {
+        const uchar4 p = px(xx, yy);
+        return f4(unorm8(p.x), unorm8(p.y), unorm8(p.z), unorm8(p.w));
+    };
     auto gray = [&](int xx, int yy) {
         if (xx < 0 || xx >= W || yy < 0 || yy >= H) return 0.0f;
         const uchar4 p = px(xx, yy);
         return gray_dot<false>(unorm8(p.x), unorm8(p.y), unorm8(p.z));
     };
-    const uchar4 p = px(x, y);
-    const float4 c = f4(unorm8(p.x), unorm8(p.y), unorm8(p.z), unorm8(p.w));
-    float4 g;
-    if (gin) {
-        g = __ldg(gin + (size_t)y * W + x);
-    } else {
-        const float dx = gray(x + 1, y) - gray(x - 1, y), dy = gray(x, y + 1) - gray(x, y - 1);
-        g = f4(dx, dy, dx, dy);
-    }
     const size_t i = (size_t)y * W + x;
-    if (compact) compact[i] = f4(c.x, c.y, c.z, __uint_as_float(sign_bytes(g)));
-    if (colour) colour[i] = c;
-    if (grad) grad[i] = g;
+    if (colour) {
+        float4 c = rgb(x, y);
+        if (r >= 0) {
+            float sum = 0.0f;
+            for (int yy = max(y - r, 0); yy <= min(y + r, H - 1); yy++)
+                for (int xx = max(x - r, 0); xx <= min(x + r, W - 1); xx++) sum += weight(rgb(xx, yy), c);
+            c.w = sum;
+        }
+        colour[i] = c;
+    }
+    if (grad) {
+        float4 g;
+        if (gin) {
+            g = __ldg(gin + i);
+        } else {
+            const float dx = gray(x + 1, y) - gray(x - 1, y), dy = gray(x, y + 1) - gray(x, y - 1);
+            g = f4(dx, dy, dx, dy);
+        }
+        grad[i] = g;
+    }
 }
 
 // vpmstereo_init / vpmstereo_init_disparity (:260-309)
@@ -255,11 +266,23 @@ __global__ void __launch_bounds__(BX* BY) k_init(float4* __restrict__ out, Views
     out[(size_t)y * V.W + x] = f4(s.x, s.y, s.z, eval<false>(V, x, y, s, n));
 }
 
+// the neighbour offsets of candidate i (:323-332): (1,0) (-1,0) (0,1) (0,-1) (16,0) (-16,0) (0,16) (0,-16), taken
+// from (iter + i) & 7: bit 2 selects the distance, bit 1 the axis, bit 0 the sign; rows and columns
+// clamped to the edge (SAMPLER_NN)
+__device__ __forceinline__ size_t neighbour(int x, int y, int k, int W, int H)
+{
+    const int d = ((k & 4) ? 16 : 1) * ((k & 1) ? -1 : 1);
+    const int ox = (k & 2) ? 0 : d, oy = (k & 2) ? d : 0;
+    return (size_t)min(max(y + oy, 0), H - 1) * W + min(max(x + ox, 0), W - 1);
+}
+
 // vpmstereo_iter_simple (:311-361).  counts (COUNT): cost-window taps, Gauss-Newton taps.
+// The general loops; not counting, it returns at once when the pair-plane kernels run.
 template <bool COUNT>
 __global__ void __launch_bounds__(BX* BY, 3) k_iter(float4* __restrict__ out, const float4* __restrict__ in, Views V,
                                                  float dmax, int iter, unsigned long long* counts)
 {
+    if (variant_skips<true>(V, !COUNT)) return;
     const int x = blockIdx.x * BX + threadIdx.x, y = blockIdx.y * BY + threadIdx.y;
     if (x >= V.W || y >= V.H) return;
     const float cx = (float)x, cy = (float)y;
@@ -268,16 +291,9 @@ __global__ void __launch_bounds__(BX* BY, 3) k_iter(float4* __restrict__ out, co
     float3 s = fronto(cx, cy, vdc2((uint32_t)((x & 7) * (y & 7)) + (uint32_t)iter) * dmax);
     float cost = eval<COUNT>(V, x, y, s, ne);
     if (cost < cur.w) cur = f4(s.x, s.y, s.z, cost);
-    // neighbour offsets (:323-332) (1,0) (-1,0) (0,1) (0,-1) (16,0) (-16,0) (0,16) (0,-16), taken
-    // from (iter + i) & 7: bit 2 selects the distance, bit 1 the axis, bit 0 the sign; rows and
-    // columns clamped to the edge (SAMPLER_NN)
 #pragma unroll 1
     for (int i = 0; i < 8; i++) {
-        const int k = (iter + i) & 7;
-        const int d = ((k & 4) ? 16 : 1) * ((k & 1) ? -1 : 1);
-        const int ox = (k & 2) ? 0 : d, oy = (k & 2) ? d : 0;
-        const int nx = min(max(x + ox, 0), V.W - 1), ny = min(max(y + oy, 0), V.H - 1);
-        const float4 n = __ldg(in + (size_t)ny * V.W + nx);
+        const float4 n = __ldg(in + neighbour(x, y, (iter + i) & 7, V.W, V.H));
         s = make_float3(n.x, n.y, n.z);
         cost = eval<COUNT>(V, x, y, s, ne);
         if (cost < cur.w) cur = f4(s.x, s.y, s.z, cost);
@@ -294,6 +310,84 @@ __global__ void __launch_bounds__(BX* BY, 3) k_iter(float4* __restrict__ out, co
     }
 }
 
+constexpr int PT = 128;   // threads of the pair-plane kernels: 4 rows of a warp each, `owners` pixels per warp
+
+// the pixel of a lane, and whether it owns one
+struct VPixel {
+    int lane, x, y;
+    bool own;
+    size_t i;
+    __device__ __forceinline__ VPixel(const Views& V, int owners)
+        : lane(threadIdx.x), x(blockIdx.x * owners + threadIdx.x), y(blockIdx.y * (PT / 32) + threadIdx.y),
+          own((int)threadIdx.x < owners && x < V.W && y < V.H), i((size_t)y * V.W + x)
+    {
+    }
+};
+
+// vpmstereo_iter_simple up to the Gauss-Newton steps (:311-345): the van der Corput candidate and the eight
+// neighbour states.  A candidate whose plane is the current one's bit for bit has its cost and cannot be below
+// it; it is skipped when the states' costs are their planes' (known; not for states from outside).
+// Bound by instruction issue, as the main path's candidate kernel; 5 blocks per SM = 96 registers.
+__global__ void __launch_bounds__(PT, 5) k_cand(float4* __restrict__ cur_out, const float4* __restrict__ in, Views V,
+                                             float dmax, int iter, int owners, int known)
+{
+    if (variant_skips<false>(V, 1)) return;
+    __shared__ WarpScratch<VPM> ws[PT / 32];
+    const VPixel P(V, owners);
+    const float cx = (float)P.x, cy = (float)P.y;
+    float4 cur = P.own ? __ldg(in + P.i) : f4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+    for (int k = 0; k < 9; k++) {
+        float4 s = cur;
+        bool need = P.own;
+        if (k == 0) {
+            const float3 f = fronto(cx, cy, vdc2((uint32_t)((P.x & 7) * (P.y & 7)) + (uint32_t)iter) * dmax);
+            s = f4(f.x, f.y, f.z, 0.0f);
+        } else if (need) {
+            s = __ldg(in + neighbour(P.x, P.y, (iter + k - 1) & 7, V.W, V.H));
+        }
+        if (known && __float_as_uint(s.x) == __float_as_uint(cur.x) && __float_as_uint(s.y) == __float_as_uint(cur.y) &&
+            __float_as_uint(s.z) == __float_as_uint(cur.z))
+            need = false;
+        s.w = patch_eval_warp<false, true, VPM>(V, ws[threadIdx.y], P.lane, need, P.x, P.y, s, cur.w);
+        if (need && s.w < cur.w) cur = s;
+    }
+    if (P.own) cur_out[P.i] = cur;
+}
+
+// three Gauss-Newton steps (:347-349), a thread per pixel or, on small images, a few pixels per warp
+template <bool SHARED>
+__global__ void __launch_bounds__(PT, 5) k_steps(float4* __restrict__ out, const float4* __restrict__ cur, Views V,
+                                              int owners)
+{
+    if (variant_skips<false>(V, 1)) return;
+    __shared__ WarpScratch<VPM> ws[SHARED ? PT / 32 : 1];
+    const VPixel P(V, owners);
+    if (SHARED) {
+        if (P.y >= V.H) return;   // a whole warp
+        float4 s = P.own ? __ldg(cur + P.i) : f4(0.0f, 0.0f, 0.0f, 0.0f);
+        s = klt2_steps_warp<false, VPM>(V, ws[threadIdx.y], P.lane, owners, 3, P.own, P.x, P.y, s);
+        if (P.own) out[P.i] = s;
+    } else if (P.own) {
+        float4 s = __ldg(cur + P.i);
+#pragma unroll 1
+        for (int k = 0; k < 3; k++) s = klt2_pair<false, VPM>(V, P.x, P.y, s);
+        out[P.i] = s;
+    }
+}
+
+// the evaluation of their result (:350-358); out holds the candidates' state
+__global__ void __launch_bounds__(PT, 5) k_settle(float4* __restrict__ out, const float4* __restrict__ steps, Views V,
+                                               int owners)
+{
+    if (variant_skips<false>(V, 1)) return;
+    __shared__ WarpScratch<VPM> ws[PT / 32];
+    const VPixel P(V, owners);
+    float4 cur = P.own ? out[P.i] : f4(0.0f, 0.0f, 0.0f, 0.0f), s = P.own ? __ldg(steps + P.i) : cur;
+    s.w = patch_eval_warp<false, true, VPM>(V, ws[threadIdx.y], P.lane, P.own, P.x, P.y, s, cur.w);
+    if (P.own && s.w < cur.w) out[P.i] = s;
+}
+
 // vpmstereo_disparity (:363-377): |x' - x| * scale
 __global__ void k_disparity(float* __restrict__ out, const float4* __restrict__ states, int W, int H, float scale)
 {
@@ -307,10 +401,20 @@ __global__ void k_disparity(float* __restrict__ out, const float4* __restrict__ 
 inline dim3 row_grid(int W, int H) { return dim3((W + 127) / 128, H); }
 inline dim3 tile_grid(int W, int H) { return dim3((W + BX - 1) / BX, (H + BY - 1) / BY); }
 
-void launch_prep(const uint8_t* img, size_t stride, int W, int H, const float4* gin, float4* compact, float4* colour,
-                 float4* grad, cudaStream_t st)
+void launch_prep(const uint8_t* img, size_t stride, int W, int H, int r, const float4* gin, float4* colour, float4* grad,
+                 cudaStream_t st)
 {
-    k_prep<<<row_grid(W, H), 128, 0, st>>>(img, stride, W, H, gin, compact, colour, grad);
+    k_prep<<<row_grid(W, H), 128, 0, st>>>(img, stride, W, H, r, gin, colour, grad);
+}
+
+// the texel planes of both images; tmp: two W*H fields
+void launch_views(float4* tex0, float4* tex1, float4* tmp0, float4* tmp1, const uint8_t* img0, const uint8_t* img1,
+                  const float4* g0, const float4* g1, int W, int H, size_t stride, int r, cudaStream_t st)
+{
+    launch_prep(img0, stride, W, H, r, g0, tmp0, tmp1, st);
+    launch_pack_tex(tex0, tmp0, tmp1, W, H, 0, st);
+    launch_prep(img1, stride, W, H, -1, g1, tmp0, tmp1, st);
+    launch_pack_tex(tex1, tmp0, tmp1, W, H, 0, st);
 }
 
 void launch_init(float4* out, const Views& V, float dmax, const float* initdisp, cudaStream_t st)
@@ -318,11 +422,21 @@ void launch_init(float4* out, const Views& V, float dmax, const float* initdisp,
     k_init<<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, V, dmax, initdisp);
 }
 
-void launch_iter(float4* out, const float4* in, const Views& V, float dmax, int iter, unsigned long long* counts,
-                 cudaStream_t st)
+// one pass from `in` to `out`; steps: a W*H field; known: every state's cost is its plane's
+void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, float dmax, int iter, int known,
+                 unsigned long long* counts, cudaStream_t st)
 {
-    if (counts) k_iter<true><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, counts);
-    else k_iter<false><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, nullptr);
+    if (counts) {
+        k_iter<true><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, counts);
+        return;
+    }
+    const int owners = prop_owners(V.W, V.H);
+    const dim3 b(32, PT / 32), g((V.W + owners - 1) / owners, (V.H + PT / 32 - 1) / (PT / 32));
+    k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known);
+    if (owners <= WARP_KLT) k_steps<true><<<g, b, 0, st>>>(steps, out, V, owners);
+    else k_steps<false><<<g, b, 0, st>>>(steps, out, V, owners);
+    k_settle<<<g, b, 0, st>>>(out, steps, V, owners);
+    k_iter<false><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, nullptr);
 }
 
 void launch_disparity(float* out, const float4* states, int W, int H, float scale, cudaStream_t st)
@@ -371,10 +485,10 @@ inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 inline bool aligned(const void* p, size_t n) { return ((uintptr_t)p % n) == 0; }
 inline size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// workspace: compact plane of image 0, colour and gradient planes of image 1, two state
-// fields, then (host entry) both images, the initial disparities, the disparities, counters
+// workspace: texel planes of both images, two state fields, the Gauss-Newton results, then (host
+// entry) both images, the initial disparities, the disparities, counters
 struct VLayout {
-    enum { t1, c2, g2, s0, s1, img0, img1, initd, disp, ctr, COUNT };
+    enum { tex0, tex1, s0, s1, steps, img0, img1, initd, disp, ctr, COUNT };
     size_t off[COUNT + 1];
     size_t total() const { return off[COUNT]; }
 };
@@ -382,7 +496,8 @@ struct VLayout {
 VLayout vlayout(int W, int H, size_t stride)
 {
     const size_t N = (size_t)W * H;
-    const size_t sz[VLayout::COUNT] = {16 * N, 16 * N, 16 * N, 16 * N, 16 * N, stride * H, stride * H, 4 * N, 4 * N, 16};
+    const size_t sz[VLayout::COUNT] = {tex_bytes(W, H), tex_bytes(W, H), 16 * N, 16 * N, 16 * N, stride * H, stride * H,
+                                        4 * N, 4 * N, 16};
     VLayout L;
     size_t o = 0;
     for (int k = 0; k < VLayout::COUNT; k++) {
@@ -429,19 +544,17 @@ int run_simple(pm_vpm* h, const uint8_t* img0, const uint8_t* img1, int W, int H
                float* disp, float4* states, cudaStream_t st)
 {
     const VLayout L = vlayout(W, H, stride);
-    float4* t1 = vat<float4>(h->ws, L, VLayout::t1);
-    float4* c2 = vat<float4>(h->ws, L, VLayout::c2);
-    float4* g2 = vat<float4>(h->ws, L, VLayout::g2);
+    float4 *tex0 = vat<float4>(h->ws, L, VLayout::tex0), *tex1 = vat<float4>(h->ws, L, VLayout::tex1);
+    float4* steps = vat<float4>(h->ws, L, VLayout::steps);
     float4* s[2] = {vat<float4>(h->ws, L, VLayout::s0), vat<float4>(h->ws, L, VLayout::s1)};
     unsigned long long* ctr = vat<unsigned long long>(h->ws, L, VLayout::ctr);
-    launch_prep(img0, stride, W, H, nullptr, t1, nullptr, nullptr, st);
-    launch_prep(img1, stride, W, H, nullptr, nullptr, c2, g2, st);
-    const Views V = {t1, c2, g2, W, H, h->patchsize};
+    launch_views(tex0, tex1, s[0], s[1], img0, img1, nullptr, nullptr, W, H, stride, h->patchsize, st);
+    const Views V = make_view(tex0, tex1, W, H, h->patchsize);
     launch_init(s[1], V, h->dmax, initdisp, st);
     if (h->counting) VPM_CUDA(h, cudaMemsetAsync(ctr, 0, 16, st));
     int swap = 0;
     for (int i = 0; i < h->iterations; i++) {
-        launch_iter(s[swap], s[1 - swap], V, h->dmax, i, h->counting ? ctr : nullptr, st);
+        launch_iter(s[swap], s[1 - swap], steps, V, h->dmax, i, 1, h->counting ? ctr : nullptr, st);
         swap = 1 - swap;
     }
     launch_disparity(disp, s[1 - swap], W, H, 1.0f, st);
@@ -454,10 +567,11 @@ int run_simple(pm_vpm* h, const uint8_t* img0, const uint8_t* img1, int W, int H
     return PM_OK;
 }
 
-// the first-image compact plane and the second image's planes from the reference kernels'
-// inputs (RGBA8 colour images and float4 gradient images), in stream-ordered scratch
+// the texel planes from the reference kernels' inputs (RGBA8 colour images and float4 gradient
+// images), in stream-ordered scratch, with a W*H field for the Gauss-Newton results
 struct VpmScratch {
     float4* p = nullptr;
+    float4* steps = nullptr;
     cudaStream_t st = nullptr;
     ~VpmScratch()
     {
@@ -467,11 +581,12 @@ struct VpmScratch {
              cudaStream_t s, Views* V)
     {
         st = s;
-        const size_t N = (size_t)W * H;
-        VPM_CUDA(nullptr, cudaMallocAsync((void**)&p, 3 * N * sizeof(float4), s));
-        launch_prep(c1, stride, W, H, reinterpret_cast<const float4*>(g1), p, nullptr, nullptr, s);
-        launch_prep(c2, stride, W, H, reinterpret_cast<const float4*>(g2), nullptr, p + N, p + 2 * N, s);
-        *V = Views{p, p + N, p + 2 * N, W, H, r};
+        const size_t N = (size_t)W * H, T = tex_bytes(W, H) / sizeof(float4);
+        VPM_CUDA(nullptr, cudaMallocAsync((void**)&p, (2 * T + 2 * N) * sizeof(float4), s));
+        steps = p + 2 * T;
+        launch_views(p, p + T, steps, steps + N, c1, c2, reinterpret_cast<const float4*>(g1),
+                     reinterpret_cast<const float4*>(g2), W, H, stride, r, s);
+        *V = make_view(p, p + T, W, H, r);
         return PM_OK;
     }
 };
@@ -588,7 +703,7 @@ int pm_k_vpm_grad(float* out, const uint8_t* img, int W, int H, size_t stride, v
     int rc = check_common(nullptr, W, H, stride, 0, 1.0f);
     if (rc) return rc;
     if (!out || !img || !aligned(out, 16) || !aligned(img, 4)) return vfail(nullptr, PM_EINVAL_ARG, "bad buffer");
-    launch_prep(img, stride, W, H, nullptr, nullptr, nullptr, reinterpret_cast<float4*>(out), S(stream));
+    launch_prep(img, stride, W, H, -1, nullptr, nullptr, reinterpret_cast<float4*>(out), S(stream));
     VPM_CUDA(nullptr, cudaGetLastError());
     return PM_OK;
 }
@@ -623,7 +738,8 @@ int pm_k_vpm_iter(float* out, const float* in, const uint8_t* c1, const float* g
     Views V;
     rc = sc.make(c1, g1, c2, g2, W, H, stride, r, S(stream), &V);
     if (rc) return rc;
-    launch_iter(reinterpret_cast<float4*>(out), reinterpret_cast<const float4*>(in), V, dmax, iter, nullptr, S(stream));
+    launch_iter(reinterpret_cast<float4*>(out), reinterpret_cast<const float4*>(in), sc.steps, V, dmax, iter, 0, nullptr,
+                S(stream));
     VPM_CUDA(nullptr, cudaGetLastError());
     return PM_OK;
 }

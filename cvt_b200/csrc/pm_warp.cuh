@@ -19,9 +19,11 @@ namespace pm {
 // 64.1; never 69.2).
 constexpr int WARP_TASKS = 16, WARP_TERMS = 16 * 23;
 
+template <Model M = PMH>
 struct WarpScratch {
     float4 par[WARP_TASKS][2];   // per pixel: plane and column of the window's left end; centre colour and top row
-    float2 term[WARP_TERMS];
+    float2 term[WARP_TERMS];     // (first part, weight) of a cost term, or (t, sc) of a Gauss-Newton term
+    float part[M == VPM ? WARP_TERMS : 1];   // second part of a cost term
 };
 
 // The items of a pass: samples e0 .. e0 + len - 1 (row by row) of n windows, item i = (task, sample e0 + i % len)
@@ -45,8 +47,8 @@ __device__ __forceinline__ int window_row(int e, unsigned recip) { return (int)(
 // Samples e0 .. e0 + len - 1 of the windows of patch_eval_census of the n pixels whose parameters are in S.par,
 // spread over the warp; their terms go to S.term[task * len + sample - e0].  ROW: all windows
 // have the top row `top` (a warp along an image row).
-template <bool F, bool ROW>
-__device__ __forceinline__ void eval_terms_shared(const ViewData& V, WarpScratch& S, int lane, int n, int e0, int len,
+template <bool F, bool ROW, Model M>
+__device__ __forceinline__ void eval_terms_shared(const ViewData& V, WarpScratch<M>& S, int lane, int n, int e0, int len,
                                                   unsigned recip, int top)
 {
     const int W = V.W, L = 2 * V.r + 1;
@@ -61,36 +63,48 @@ __device__ __forceinline__ void eval_terms_shared(const ViewData& V, WarpScratch
         const float4 q = __ldg(V.row1c(yc) + min(max(x, 0), W - 1));
         const float p2x = match<F>(A, qx, A.y * (float)y);
         const float t = fminf(fmaxf((p2x + 0.5f) - 0.5f, 0.0f), fW);   // in [0, W], 0 for a NaN
-        float w = support_weight<F>(q.x - B.x, q.y - B.y, q.z - B.z);
+        float w = pair_support<F, M>(q.x - B.x, q.y - B.y, q.z - B.z);
         const uintptr_t base = reinterpret_cast<uintptr_t>(V.row2p(yc)) - (uintptr_t)0x4B000000u * 16u;
         PairSigns d;
         float a;
-        float cost = eval_sample_pair<F>(base, q, t, d, a);
+        float ad = eval_sample_pair<F>(base, q, t, d, a);
         int nm = pair_mismatch(d, __float_as_uint(q.w));
         // a NaN column reads the positive quiet NaN: full colour cost, positive signs
         const bool nan = p2x != p2x;
         if (unsure(unsure_max(0u, d)) || nan) {
             nm = nan ? sign_mismatch(__float_as_uint(q.w), 0u)
                      : exact_mismatch<F>(V.row2(yc) + V.plane + (int)t, a, __float_as_uint(q.w));
-            if (nan) cost = PM_K033_8 * 3.0f;
+            if (nan) ad = 3.0f;
         }
-        cost = fmaf(0.21875f, (float)nm, cost);
         if (!in1 || p2x < 0.0f || p2x >= fW) w = 0.0f;
-        S.term[it.i] = f2(F ? cost : w * cost, w);
+        const SampleTerms c = sample_terms<F, M>(w, ad, nm);
+        S.term[it.i] = f2(c.a, w);
+        if (M == VPM) S.part[it.i] = c.b;
     }
 }
 
 // patch_eval_census (:661-736) for the pixels of a warp whose lanes set `need`; all 32 lanes call.
 // S: this warp's scratch.  All windows of the warp are at the same sample e0: rows that the lanes run on
 // their own end on a whole row, and once few enough windows are left they stay shared.
-template <bool F, bool ROW>
-__device__ __forceinline__ float patch_eval_warp(const ViewData& V, WarpScratch& S, int lane, bool need, int px, int py,
+//
+// VPM (VPMStereo.cl:200-258) has no early exit of its own, but its caller only asks whether the cost is below
+// mincost.  The census only grows and the weight sum stays at or below the whole window's
+// (in.w; sums of a subset of the terms in the same order round no higher), so once
+// census / in.w >= mincost the cost cannot be below mincost any more, and any such value may be returned.
+template <bool F, bool ROW, Model M = PMH>
+__device__ __forceinline__ float patch_eval_warp(const ViewData& V, WarpScratch<M>& S, int lane, bool need, int px, int py,
                                                  float4 s, float mincost)
 {
     const float cx = (float)px, cy = (float)py;
-    float ret = 1e5f, wsum = 0.0f, census = 0.0f, thr = 0.0f;
+    float ret = M == PMH ? 1e5f : 1.0f, wsum = 0.0f, census = 0.0f, thr = 0.0f;
     float4 in = f4(0.0f, 0.0f, 0.0f, 0.0f);
-    bool act = need && plane_usable(s, cx, cy, V.W);
+    bool act = need;
+    if (M == PMH) {
+        act = act && plane_usable(s, cx, cy, V.W);
+    } else {
+        const float c2x = transform_x(s, cx, cy);
+        act = act && !(c2x < 0 || c2x >= (float)V.W);
+    }
     if (act) {
         in = __ldg(V.row1(py) + px);
         thr = exit_threshold(mincost, in.w);
@@ -104,7 +118,7 @@ __device__ __forceinline__ float patch_eval_warp(const ViewData& V, WarpScratch&
         if (n == 0) break;
         if (n > WARP_TASKS) {   // every lane its own row
             const int iy = top + window_row(e0, recip);
-            if (act && iy >= 0 && iy < V.H) eval_row_pixel<F>(V, iy, s, s.y * (float)iy, in, qx0, qx1, census, wsum);
+            if (act && iy >= 0 && iy < V.H) eval_row_pixel<F, M>(V, iy, s, s.y * (float)iy, in, qx0, qx1, census, wsum);
             e0 += L;
         } else {
             const int rank = __popc(m & ((1u << lane) - 1u));
@@ -114,38 +128,37 @@ __device__ __forceinline__ float patch_eval_warp(const ViewData& V, WarpScratch&
                 S.par[rank][1] = f4(in.x, in.y, in.z, __int_as_float(top));
             }
             __syncwarp();
-            eval_terms_shared<F, ROW>(V, S, lane, n, e0, len, recip, top);
+            eval_terms_shared<F, ROW, M>(V, S, lane, n, e0, len, recip, top);
             __syncwarp();
             if (act) {
                 const float2* v = S.term + rank * len;
 #pragma unroll 4
                 for (int k = 0; k < len; k++) {
                     const float2 c = v[k];
-                    census = F ? fmaf(c.y, c.x, census) : census + c.x;
-                    wsum += c.y;
+                    add_terms<F, M>(census, wsum, c.y, SampleTerms{c.x, M == VPM ? S.part[rank * len + k] : 0.0f});
                 }
             }
             e0 += len;
             __syncwarp();
         }
         if (act && census >= thr && wsum > 0.0f) {   // the exit test, as in patch_eval_pair
-            ret = 1.0f;
+            ret = M == PMH ? 1.0f : __int_as_float(0x7f800000);
             act = false;
         }
     }
-    if (act) ret = wsum <= 1.0f ? 1.1f : census / wsum;
+    if (act) ret = M == PMH && wsum <= 1.0f ? 1.1f : census / wsum;
     return ret;
 }
 
-// Six steps of patch_census_klt2 (:326-410) for the first `owners` <= WARP_KLT lanes of a warp along an image
+// `steps` steps of patch_census_klt2 (:326-410) for the first `owners` <= WARP_KLT lanes of a warp along an image
 // row, those with `need`; all 32 lanes call.  The terms (t, sc) of all owned windows are
 // spread over the lanes, pass by pass; each of a window's nine sums belongs to one lane, which
 // adds its products in sample order.  The factor of a sum is a product of two of 1, qx, qy, exact.
 constexpr int WARP_KLT = 4;
 static_assert(WARP_KLT <= WARP_TASKS, "klt2_steps_warp keeps its pixels in the scratch");
-template <bool F>
-__device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch& S, int lane, int owners, bool need, int px,
-                                                  int py, float4 s)
+template <bool F, Model M = PMH>
+__device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch<M>& S, int lane, int owners, int steps,
+                                                  bool need, int px, int py, float4 s)
 {
     constexpr int NU = (9 * WARP_KLT + 31) / 32;   // sums per lane, at most
     const int W = V.W, r = V.r, L = 2 * r + 1, top = py - r;
@@ -156,7 +169,7 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
     float* const sums = reinterpret_cast<float*>(S.term);
     const float4 c1 = need ? __ldg(V.row1(py) + px) : f4(0.0f, 0.0f, 0.0f, 0.0f);
     const int chunk = WARP_TERMS / owners;
-    for (int step = 0; step < 6; step++) {
+    for (int step = 0; step < steps; step++) {
         // a NaN plane has no column: no sample counts, the 0 / 0 solution is NaN
         const bool nan = s.x != s.x || s.y != s.y || s.z != s.z;
         const unsigned m = __ballot_sync(0xffffffffu, need && !nan);
@@ -178,7 +191,7 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
                 // the 3-point cost needs 1 <= qx < W - 1
                 if (((m >> it.task) & 1u) && qx >= 1.0f && qx < (float)(W - 1)) {
                     const float4 c = S.par[it.task][1];
-                    klt_terms<F, false, false>(W, V.row2p(y), V.row2(y) + V.plane, __ldg(V.row1c(y) + (int)qx), c,
+                    klt_terms<F, false, false, M>(W, V.row2p(y), V.row2(y) + V.plane, __ldg(V.row1c(y) + (int)qx), c,
                                                match<F>(A, qx, A.y * (float)y), v.x, v.y);
                 }
                 S.term[it.i] = v;

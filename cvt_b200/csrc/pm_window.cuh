@@ -422,6 +422,40 @@ __device__ __forceinline__ float4 klt2_general(const ViewData& V, int px, int py
 }
 
 // ---- pair-plane loops ------------------------------------------------------------------
+//
+// The loops serve two window models, their last template parameter: PMH, the functions of pmhstereo.cl
+// that the comments cite, and VPM, those of VPMStereo.cl (patch_eval_census :200-258, patch_census_klt
+// :117-198; pm_vpm.cu), which differ in the support weight, the mix of the two costs, the reference colour
+// of a Gauss-Newton tap and in taking every Gauss-Newton sample.
+enum Model { PMH, VPM };
+
+// support weight of a colour difference
+template <bool F, Model M>
+__device__ __forceinline__ float pair_support(float dx, float dy, float dz)
+{
+    return expf_neg(-fabsf(gray_dot<F>(dx, dy, dz)) * (M == PMH ? 12.0f : 8.0f));
+}
+
+// the two parts of a sample's weighted cost, PMH: their sum (one product), VPM: colour and census part
+struct SampleTerms {
+    float a, b;
+};
+template <bool F, Model M>
+__device__ __forceinline__ SampleTerms sample_terms(float w, float ad, int n)
+{
+    if (M == VPM) return SampleTerms{w * 0.05f * 0.33f * ad, w * (1.0f - 0.05f) * 0.25f * (float)n};
+    // K ad + 0.875f * (0.25f * n): the product 0.21875 n is exact, so one fma rounds the same
+    const float cost = fmaf(0.21875f, (float)n, PM_K033_8 * ad);
+    return SampleTerms{F ? cost : w * cost, 0.0f};
+}
+// adds a sample to the sums
+template <bool F, Model M>
+__device__ __forceinline__ void add_terms(float& census, float& wsum, float w, SampleTerms s)
+{
+    if (M == VPM) census = (census + s.a) + s.b;
+    else census = F ? fmaf(w, s.a, census) : census + s.a;
+    wsum += w;
+}
 
 // byte K of a record word / 255, correctly rounded, in one permute and one fma: the byte twice, in bits
 // 8-23 of an otherwise zero word, is x = 257 byte 2^-141 as a float (exponent field 0 or 1, one
@@ -504,8 +538,8 @@ __device__ __forceinline__ float match(float4 s, float qx, float byq)
 }
 
 // One sample of patch_eval_census (:690-722): compact texel q of the first view, matched column p2x whose
-// t = (p2x + 0.5) - 0.5 lies in [0, W], weight w.  The column's texel is at base + 16 * (bits of the float
-// 2^23 + column).  Returns the sample's cost and the signs.
+// t = (p2x + 0.5) - 0.5 lies in [0, W].  The column's texel is at base + 16 * (bits of the float
+// 2^23 + column).  Returns the sample's colour cost (ad_sum) and the signs.
 template <bool F>
 __device__ __forceinline__ float eval_sample_pair(uintptr_t base, float4 q, float t, PairSigns& d, float& a)
 {
@@ -517,12 +551,12 @@ __device__ __forceinline__ float eval_sample_pair(uintptr_t base, float4 q, floa
     float ad = trunc_ad(mix<F>(a, b1, pair_unit<0>(R.x), pair_unit<0>(R.y)) - q.x);
     ad = ad + trunc_ad(mix<F>(a, b1, pair_unit<1>(R.x), pair_unit<1>(R.y)) - q.y);
     ad = ad + trunc_ad(mix<F>(a, b1, pair_unit<2>(R.x), pair_unit<2>(R.y)) - q.z);
-    return PM_K033_8 * ad;
+    return ad;
 }
 
 // a row of patch_eval_pair.  IN: every matched column lies in the image; otherwise all are finite and
 // samples outside get weight 0.  SURE: no sign can be unsure; otherwise returns unsure_max.
-template <bool F, bool IN, bool SURE>
+template <bool F, bool IN, bool SURE, Model M>
 __device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, uintptr_t base, const float4* __restrict__ q1,
                                              float4 in, float4 s, float byq, float qx0, float qx1, float fW)
 {
@@ -532,16 +566,13 @@ __device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, uintptr
         const float p2x = match<F>(s, qx, byq);
         float t = (p2x + 0.5f) - 0.5f;
         if (!IN) t = fminf(fmaxf(t, 0.0f), fW);
-        float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
+        float w = pair_support<F, M>(q.x - in.x, q.y - in.y, q.z - in.z);
         if (!IN) w = p2x >= 0.0f && p2x < fW ? w : 0.0f;
         PairSigns d;
         float a;
-        float cost = eval_sample_pair<F>(base, q, t, d, a);
+        const float ad = eval_sample_pair<F>(base, q, t, d, a);
         if (!SURE) m = unsure_max(m, d);
-        // cost + 0.875f * (0.25f * n): the product 0.21875 n is exact, so one fma rounds the same
-        cost = fmaf(0.21875f, (float)pair_mismatch(d, __float_as_uint(q.w)), cost);
-        census = F ? fmaf(w, cost, census) : census + w * cost;
-        wsum += w;
+        add_terms<F, M>(census, wsum, w, sample_terms<F, M>(w, ad, pair_mismatch(d, __float_as_uint(q.w))));
     }
     return m;
 }
@@ -551,7 +582,7 @@ __device__ __forceinline__ uint32_t eval_row(float& census, float& wsum, uintptr
 // non-finite.  From column 256 on a tap weight is a multiple of 2^-15 and no sign is unsure.
 // Rows with a non-finite column and rows where some sign was unsure run sample by sample with the
 // signs from the gradients.
-template <bool F>
+template <bool F, Model M = PMH>
 __device__ __forceinline__ void eval_row_pixel(const ViewData& V, int iy, float4 s, float byq, float4 in, float qx0,
                                                float qx1, float& census, float& wsum)
 {
@@ -566,13 +597,13 @@ __device__ __forceinline__ void eval_row_pixel(const ViewData& V, int iy, float4
     const unsigned lanes = __activemask();
     bool single = true;
     if (__all_sync(lanes, sure)) {
-        eval_row<F, true, true>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW);
+        eval_row<F, true, true, M>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW);
         single = false;
     } else if (__all_sync(lanes, in_image)) {
-        single = unsure(eval_row<F, true, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
+        single = unsure(eval_row<F, true, false, M>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
     } else if (__all_sync(lanes, fin(pa) && fin(pb))) {
         if (!__any_sync(lanes, plo < fW && phi >= 0.0f)) return;
-        single = unsure(eval_row<F, false, false>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
+        single = unsure(eval_row<F, false, false, M>(census, wsum, base, q1, in, s, byq, qx0, qx1, fW)) && !sure;
     }
     if (!single) return;
     census = census0;
@@ -582,19 +613,17 @@ __device__ __forceinline__ void eval_row_pixel(const ViewData& V, int iy, float4
         const float p2x = match<F>(s, qx, byq);
         if (p2x < 0 || p2x >= fW) continue;
         const float4 q = __ldg(q1);
-        const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
-        float cost;
+        const float w = pair_support<F, M>(q.x - in.x, q.y - in.y, q.z - in.z);
+        float ad = 3.0f;   // a NaN column reads the positive quiet NaN: full colour cost, positive signs
+        int nm = sign_mismatch(__float_as_uint(q.w), 0u);
         if (p2x == p2x) {
             PairSigns d;
             float a;
             const float t = (p2x + 0.5f) - 0.5f;
-            cost = eval_sample_pair<F>(base, q, t, d, a);
-            cost = fmaf(0.21875f, (float)exact_mismatch<F>(g2 + (int)t, a, __float_as_uint(q.w)), cost);
-        } else {   // a NaN column reads the positive quiet NaN: full colour cost, positive signs
-            cost = fmaf(0.21875f, (float)sign_mismatch(__float_as_uint(q.w), 0u), PM_K033_8 * 3.0f);
+            ad = eval_sample_pair<F>(base, q, t, d, a);
+            nm = exact_mismatch<F>(g2 + (int)t, a, __float_as_uint(q.w));
         }
-        census = F ? fmaf(w, cost, census) : census + w * cost;
-        wsum += w;
+        add_terms<F, M>(census, wsum, w, sample_terms<F, M>(w, ad, nm));
     }
 }
 
@@ -620,10 +649,10 @@ __device__ __forceinline__ float patch_eval_pair(const ViewData& V, int px, int 
     return census / wsum;
 }
 
-// The cost of a Gauss-Newton tap, k1 * ad + x * 0.25 * n (:361-370).  The source's sum is a double
+// The cost of a Gauss-Newton tap, k1 * ad + x * 0.25 * n (:361-370; VPMStereo.cl:154-162).  The source's sum is a double
 // one rounded to float; here one fma.  They agree for colours k / 255: a nonzero truncated difference is
 // then >= 2^-33 (the reference colour is 0 or >= 2^-8 in magnitude, the tap weights are multiples
-// of 2^-25), so the colour term is 0 or >= 2^-34 of the weight; the double sum is inexact only when
+// of 2^-25), so the colour term is 0 or >= 2^-36 of the weight; the double sum is inexact only when
 // the colour term is below 2^-28 of the sum, and then it cannot land on a midpoint of two floats
 // unless the colour term is below 2^-53 of it.
 __device__ __forceinline__ float tap_cost(float k1, float x, float ad, int n) { return fmaf(x, (float)n, k1 * ad); }
@@ -674,7 +703,7 @@ __device__ __forceinline__ float tap_alone(float u, int W, const float4* __restr
 // is clamped to the padded row, where records beyond the image hold edge texels, as the
 // source's clamp gives.  Where a weight is out of range (floors that do not chain, a non-finite column) or,
 // not SURE, a sign unsure, each tap is read on its own.
-template <bool F, bool EVEN, bool SURE>
+template <bool F, bool EVEN, bool SURE, Model M>
 __device__ __forceinline__ void klt_terms(int W, const float4* __restrict__ row2, const float4* __restrict__ g2, float4 q,
                                           float4 c1, float p2x, float& t, float& sc)
 {
@@ -697,9 +726,13 @@ __device__ __forceinline__ void klt_terms(int W, const float4* __restrict__ row2
     const uint32_t A0 = pair_weight(a0), Am = EVEN ? A0 : pair_weight(am), Ap = EVEN ? A0 : pair_weight(ap);
     const uint32_t sb1 = __float_as_uint(q.w);
     const PairSigns dm = pair_signs(Am, Rm), d0 = pair_signs(A0, R0), dp = pair_signs(Ap, Rp);
-    const float3 nref = make_float3(c1.x - q.x, c1.y - q.y, c1.z - q.z);   // minus the colour difference
-    float w1 = support_weight<F>(nref.x, nref.y, nref.z);
-    const float k1 = w1 * PM_K033_8, x = w1 * 0.21875f;   // (w1 * 0.875f) * 0.25, exact scaling
+    const float3 df = make_float3(c1.x - q.x, c1.y - q.y, c1.z - q.z);
+    float w1 = pair_support<F, M>(df.x, df.y, df.z);
+    // minus the reference colour: PMH takes the colour difference (:352, :364), VPM the colour
+    const float3 nref = M == PMH ? df : make_float3(-q.x, -q.y, -q.z);
+    const float k1 = M == PMH ? w1 * PM_K033_8 : w1 * 0.05f * 0.33f;
+    // (w1 * 0.875f) * 0.25, (w1 * 0.95f) * 0.25: exact scaling
+    const float x = M == PMH ? w1 * 0.21875f : w1 * (1.0f - 0.05f) * 0.25f;
     const float b0 = 1.0f - a0, bm = EVEN ? b0 : 1.0f - am, bp = EVEN ? b0 : 1.0f - ap;
     const float3 tA = pair_rgb(Rm.x), tB = pair_rgb(R0.x);
     float Cm = tap_cost(k1, x, tap_ad<F>(tA, tB, am, bm, nref), pair_mismatch(dm, sb1));
@@ -720,13 +753,13 @@ __device__ __forceinline__ void klt_terms(int W, const float4* __restrict__ row2
     }
     // the update of :394-402 without a branch
     const float curv = fmaf(-2.0f, C, Cp + Cm);   // 2 C is exact
-    const float wt = curv > 0.0f ? w1 : 0.0f;
+    const float wt = M == VPM || curv > 0.0f ? w1 : 0.0f;
     t = wt * (Cm - Cp);
     sc = wt * curv;
 }
 
 // a row of klt2_pair
-template <bool F, bool EVEN, bool SURE>
+template <bool F, bool EVEN, bool SURE, Model M>
 __device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restrict__ row2, const float4* __restrict__ g2,
                                         const float4* __restrict__ q1, float4 c1, float4 s, float byq, float qx0, float qx1,
                                         float qy)
@@ -734,7 +767,7 @@ __device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restr
     const float yy = qy * qy;
     for (float qx = qx0; qx <= qx1; qx += 1.0f, q1++) {
         float t, sc;
-        klt_terms<F, EVEN, SURE>(W, row2, g2, __ldg(q1), c1, match<F>(s, qx, byq), t, sc);
+        klt_terms<F, EVEN, SURE, M>(W, row2, g2, __ldg(q1), c1, match<F>(s, qx, byq), t, sc);
         if (F) {
             A.J0 = fmaf(t, qx, A.J0);
             A.J1 = fmaf(t, qy, A.J1);
@@ -759,7 +792,7 @@ __device__ __forceinline__ void klt_row(KltSums& A, int W, const float4* __restr
 
 // patch_census_klt2 (:326-410) over pair records.  p2x is monotone along a row, so its two ends decide
 // the row's kind (klt_row), for the warp: one whose lanes differ would run several loops.
-template <bool F>
+template <bool F, Model M = PMH>
 __device__ __forceinline__ float4 klt2_pair(const ViewData& V, int px, int py, float4 s)
 {
     // a NaN plane has no column: no sample counts, the 0 / 0 solution is NaN
@@ -782,10 +815,10 @@ __device__ __forceinline__ float4 klt2_pair(const ViewData& V, int px, int py, f
         const bool even = pa >= 1.0f && pb >= 1.0f && phi < 4194304.0f &&
                           ((__float_as_uint(phi + 1.5f) ^ __float_as_uint(plo)) < 0x00800000u);
         const unsigned lanes = __activemask();
-        if (!__all_sync(lanes, even)) klt_row<F, false, false>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
+        if (!__all_sync(lanes, even)) klt_row<F, false, false, M>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
         // from column 256 on the weight is a multiple of 2^-15 and no sign is unsure
-        else if (__all_sync(lanes, plo >= 256.0f)) klt_row<F, true, true>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
-        else klt_row<F, true, false>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
+        else if (__all_sync(lanes, plo >= 256.0f)) klt_row<F, true, true, M>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
+        else klt_row<F, true, false, M>(A, V.W, row2, g2, q1, c1, s, byq, qx0, qx1, qy);
     }
     const float3 d = lusolve(A.h00, A.h01, A.h02, A.h11, A.h12, A.h22, make_float3(A.J0 * 0.5f, A.J1 * 0.5f, A.J2 * 0.5f));
     return f4(s.x - d.x, s.y - d.y, s.z - d.z, s.w - 1e5f);

@@ -94,6 +94,28 @@ def test_vpm_kernels_match_reference_golden(torch_cuda, native, case):
     assert bits_equal(k.disparity(g["k_iter5"], 1.0 / dmax), g["k_disp_scaled"]).all()
 
 
+@pytest.mark.parametrize("finite", [True, False])
+@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 3), (149, 80, 4)])
+def test_vpm_iteration_over_pair_planes_matches_oracle(torch_cuda, native, orc, W, H, r, finite):
+    """One pass from the planes of pair_planes with costs that are not the planes': two, four and 32 pixels per
+    warp; with first-image gradients that are not finite, the general loops.  (Infinite second-image gradients
+    interpolate to NaNs, whose sign is the machine's.)"""
+    from test_gpu_parity import pair_planes
+
+    rng = np.random.default_rng(11 * W + r)
+    L = rng.integers(0, 256, (H, W, 4), dtype=np.uint8)
+    R = np.clip(np.roll(L, -2, 1).astype(int) + rng.integers(-9, 10, L.shape), 0, 255).astype(np.uint8)
+    g0, g1 = orc.vpm_grad(L), orc.vpm_grad(R)
+    P = pair_planes(rng, W, H, g1)
+    P[..., 3] = rng.choice(np.array([0.0, 0.1, 0.3, 1.0, -1.0, 5.0, np.inf], np.float32), (H, W))
+    if not finite:
+        g0[rng.random((H, W)) < 0.1] = -np.inf
+        g0[0, 0] = np.nan
+    for it in (0, 3):
+        got = K(torch_cuda, native).iter(P, L, g0, R, g1, r, 16.0, it)
+        assert bits_equal(got, orc.vpm_iter(P, L, g0, R, g1, r, 16.0, it)).all()
+
+
 @pytest.mark.parametrize("case", vpm_cases())
 def test_vpm_disparity_simple_matches_reference_golden(torch_cuda, native, case):
     """host and device entries of disparitySimple"""
