@@ -18,6 +18,12 @@
 // the reference reads and writes the cells in one barrier interval, which OpenCL leaves
 // undefined.
 //
+// The second frame is read at flow-displaced points, four texels per bilinear tap: the quad plane holds the
+// four as bytes in one 16-byte record, one gather per tap where the float texels took four, which
+// kept the L1 86% busy at 54% of the issue slots.  A colour byte / 255 takes one permute and one fma
+// (pair_unit).  A candidate that the pull alone rules out is not evaluated, one whose cost can no longer
+// win is dropped, and a warp shares the windows it has left when they are few (k_prop).
+//
 // Arithmetic is the reference's FP32 sequence (-fmad=false): every result equals the
 // restatement in oracle/pm_oracle.cpp bit for bit.  log, sin and cos are the library's own
 // (pm_math.cuh), as in the oracle.
@@ -29,7 +35,7 @@
 #include <string>
 
 #include "../../include/cvtpm.h"
-#include "pm_device.cuh"
+#include "pm_warp.cuh"
 
 namespace pm {
 namespace svpm {
@@ -40,8 +46,10 @@ constexpr int BUF = G + 2 * OFF;
 constexpr int PB = G + 2;      // dual buffer: the group and a 1-pixel apron
 
 struct Frames {
-    const float4* __restrict__ c1;   // first frame, k / 255
-    const float4* __restrict__ c2;   // second frame
+    const float4* __restrict__ c1;    // first frame, k / 255, and the window's weight sum
+    const float4* __restrict__ c2;    // second frame, k / 255
+    const uint4* __restrict__ quad;   // second frame: the RGBA8 texels (i, j), (i + 1, j), (i, j + 1), (i + 1, j + 1),
+                                      // clamped to the frame, for 0 <= i <= W, 0 <= j <= H, rows of W + 1
     int W, H, r;
 };
 
@@ -101,6 +109,127 @@ __device__ float eval(const Frames& F, int x, int y, float fx, float fy, unsigne
     return ret / wsum;
 }
 
+// support weight of a first-frame colour (:191-193); the argument lies in [-7.8001, 0]
+__device__ __forceinline__ float weight(float4 vc, float4 v1)
+{
+    return expf_neg(-((fabsf(vc.x - v1.x) + fabsf(vc.y - v1.y)) + fabsf(vc.z - v1.z)) * 2.6f);
+}
+
+// the truncated absolute difference of a tap (:195-198) at 0 <= u <= W in the row whose records start at `row`,
+// with vertical weights b, 1 - b: bilinear() of the four texels, minus the first frame's colour
+__device__ __forceinline__ float tap_sad(const uint4* __restrict__ row, float u, float b, float b1, float4 v1)
+{
+    const float fm = __fadd_rd(u, 8388608.0f);   // 2^23 + floor(u)
+    const float a = u - (fm - 8388608.0f), a1 = 1.0f - a;
+    const uintptr_t base = reinterpret_cast<uintptr_t>(row) - (uintptr_t)0x4B000000u * 16u;
+    const uint4 R = __ldg(reinterpret_cast<const uint4*>(base + (uintptr_t)__float_as_uint(fm) * 16u));
+    const float w00 = a1 * b1, w10 = a * b1, w01 = a1 * b, w11 = a * b;
+    const float x = ((w00 * pair_unit<0>(R.x) + w10 * pair_unit<0>(R.y)) + w01 * pair_unit<0>(R.z)) + w11 * pair_unit<0>(R.w);
+    const float y = ((w00 * pair_unit<1>(R.x) + w10 * pair_unit<1>(R.y)) + w01 * pair_unit<1>(R.z)) + w11 * pair_unit<1>(R.w);
+    const float z = ((w00 * pair_unit<2>(R.x) + w10 * pair_unit<2>(R.y)) + w01 * pair_unit<2>(R.z)) + w11 * pair_unit<2>(R.w);
+    return (fminf(fabsf(v1.x - x), 0.02f) + fminf(fabsf(v1.y - y), 0.02f)) + fminf(fabsf(v1.z - z), 0.02f);
+}
+
+// a row of the window on its own lane; IN: every tap's column lies in the second frame, otherwise taps
+// outside get weight 0
+template <bool IN>
+__device__ __forceinline__ void eval_row(const Frames& F, const float4* __restrict__ v, const uint4* __restrict__ row,
+                                         float x0, float x1, float fx, float b, float b1, float4 vc, float& ret, float& wsum)
+{
+    const float fW = (float)F.W;
+    for (float px = x0; px <= x1; px += 1.0f, v++) {
+        const float4 v1 = __ldg(v);
+        const float qx = px + fx;
+        float u = (qx + 0.5f) - 0.5f;
+        float w = weight(vc, v1);
+        if (!IN) {
+            u = fminf(fmaxf(u, 0.0f), fW);
+            w = qx < 0 || qx >= fW ? 0.0f : w;
+        }
+        ret += w * tap_sad(row, u, b, b1, v1);
+        wsum += w;
+    }
+}
+
+// svpmflow_eval_bilateral_trunc_sad (SVPMFlow.cl:170-209) for the pixels of a warp whose lanes set `need` (finite
+// flows); all 32 lanes call.  The sum of the truncated differences only grows and the weight sum stays at
+// or below the whole window's, so a cost that has passed `most` cannot fall below it; infinity is
+// returned then.  From 16 windows down their taps are spread over the warp and added in order by
+// the lanes that own them (patch_eval_warp).
+__device__ __forceinline__ float eval_warp(const Frames& F, WarpScratch<>& S, int lane, bool need, int x, int y, float fx,
+                                           float fy, float most)
+{
+    const int W = F.W, H = F.H, r = F.r, L = 2 * r + 1;
+    const float fW = (float)W, fH = (float)H;
+    const bool inside = x < W && y < H;
+    float4 vc = f4(0.0f, 0.0f, 0.0f, 0.0f);
+    float thr = 0.0f, ret = 0.0f, wsum = 0.0f, cost = 0.0f;
+    if (need) {
+        vc = __ldg(F.c1 + (size_t)min(y, H - 1) * W + min(x, W - 1));
+        // past rounding: cost > most follows from the sum over the whole window's weights
+        thr = inside ? most * vc.w * 1.00002f : __int_as_float(0x7f800000);
+    }
+    const float x0 = (float)max(x - r, 0), x1 = (float)min(x + r, W - 1);
+    const unsigned recip = ((1u << 20) + L - 1) / L;
+    bool act = need;
+    for (int e0 = 0; e0 < L * L;) {
+        const unsigned m = __ballot_sync(0xffffffffu, act);
+        const int n = __popc(m);
+        if (n == 0) break;
+        if (n > WARP_TASKS) {
+            const int iy = y - r + window_row(e0, recip);
+            const float qy = (float)iy + fy;
+            if (act && iy >= 0 && iy < H && !(qy < 0 || qy >= fH)) {
+                const float v = (qy + 0.5f) - 0.5f, fv = floorf(v), b = v - fv;
+                const uint4* row = F.quad + (size_t)(int)fv * (W + 1);
+                const float4* v1 = F.c1 + (size_t)iy * W + (int)x0;
+                const bool in = x0 + fx >= 0 && x1 + fx < fW;
+                if (__all_sync(__activemask(), in)) eval_row<true>(F, v1, row, x0, x1, fx, b, 1.0f - b, vc, ret, wsum);
+                else eval_row<false>(F, v1, row, x0, x1, fx, b, 1.0f - b, vc, ret, wsum);
+            }
+            e0 += L;
+        } else {
+            const int rank = __popc(m & ((1u << lane) - 1u));
+            const int len = min((WARP_TERMS / n - 1) | 1, L * L - e0);
+            if (act) {
+                S.par[rank][0] = f4(fx, fy, __int_as_float(x - r), __int_as_float(y - r));
+                S.par[rank][1] = vc;
+            }
+            __syncwarp();
+            for (WarpItem it(lane, e0, len); it.i < n * len; it.next()) {
+                const float4 A = S.par[it.task][0], c = S.par[it.task][1];
+                const int e = it.e0 + it.e, j = window_row(e, recip);
+                const int iy = __float_as_int(A.w) + j, ix = __float_as_int(A.z) + e - j * L;
+                const float qx = (float)ix + A.x, qy = (float)iy + A.y;
+                const bool in = (unsigned)ix < (unsigned)W && (unsigned)iy < (unsigned)H && !(qx < 0 || qx >= fW) &&
+                                !(qy < 0 || qy >= fH);
+                const float u = fminf(fmaxf((qx + 0.5f) - 0.5f, 0.0f), fW), v = fminf(fmaxf((qy + 0.5f) - 0.5f, 0.0f), fH);
+                const float fv = floorf(v), b = v - fv;
+                const float4 v1 = __ldg(F.c1 + (size_t)min(max(iy, 0), H - 1) * W + min(max(ix, 0), W - 1));
+                const float w = in ? weight(c, v1) : 0.0f;
+                S.term[it.i] = f2(w * tap_sad(F.quad + (size_t)(int)fv * (W + 1), u, b, 1.0f - b, v1), w);
+            }
+            __syncwarp();
+            if (act) {
+                const float2* t = S.term + rank * len;
+#pragma unroll 4
+                for (int k = 0; k < len; k++) {
+                    ret += t[k].x;
+                    wsum += t[k].y;
+                }
+            }
+            e0 += len;
+            __syncwarp();
+        }
+        if (act && ret > thr) {
+            cost = __int_as_float(0x7f800000);
+            act = false;
+        }
+    }
+    if (act) cost = wsum < 1.1f ? 1e5f : ret / wsum;
+    return cost;
+}
+
 // box_mueller (SVPMFlow.cl:38-46); theta = 2.0f * M_PI * y is a double product (M_PI is a double)
 __device__ __forceinline__ float2 box_mueller(Rng& g)
 {
@@ -130,13 +259,36 @@ __device__ __forceinline__ float2 state_refine(Rng& g, float refinemax)
 // RNG_init(&rng, linpos, k): skip distance (linpos) * k as an int (RNG.cl:54-57)
 __device__ __forceinline__ int skip(int linpos, int k) { return (int)((uint32_t)linpos * (uint32_t)k); }
 
-// the colour planes of a frame: k / 255 per channel
+// the colour plane of a frame: k / 255 per channel
 __global__ void k_colour(const uint8_t* __restrict__ img, size_t stride, int W, int H, float4* __restrict__ out)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;
     const uchar4 p = __ldg(reinterpret_cast<const uchar4*>(img + (size_t)y * stride) + x);
     out[(size_t)y * W + x] = f4(unorm8(p.x), unorm8(p.y), unorm8(p.z), unorm8(p.w));
+}
+
+// the window's weight sum, in the first frame's w component (the other components are only read)
+__global__ void k_weight_sum(float4* c1, int W, int H, int r)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x >= W) return;
+    const float4 vc = c1[(size_t)y * W + x];
+    float sum = 0.0f;
+    for (int iy = max(y - r, 0); iy <= min(y + r, H - 1); iy++)
+        for (int ix = max(x - r, 0); ix <= min(x + r, W - 1); ix++) sum += weight(vc, c1[(size_t)iy * W + ix]);
+    reinterpret_cast<float*>(c1 + (size_t)y * W + x)[3] = sum;
+}
+
+// the quad plane of the second frame (Frames)
+__global__ void k_quad(const uint8_t* __restrict__ img, size_t stride, int W, int H, uint4* __restrict__ out)
+{
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
+    if (x > W) return;
+    const uint32_t* r0 = reinterpret_cast<const uint32_t*>(img + (size_t)min(y, H - 1) * stride);
+    const uint32_t* r1 = reinterpret_cast<const uint32_t*>(img + (size_t)min(y + 1, H - 1) * stride);
+    const int x0 = min(x, W - 1), x1 = min(x + 1, W - 1);
+    out[(size_t)y * (W + 1) + x] = make_uint4(__ldg(r0 + x0), __ldg(r0 + x1), __ldg(r1 + x0), __ldg(r1 + x1));
 }
 
 // svpmflow_init (:213-233)
@@ -154,11 +306,18 @@ __global__ void __launch_bounds__(G* G) k_init(float4* __restrict__ out, Frames 
 // svpmflow_prop_local_tv_admm (:574-731), one CTA per 16x16 work-group.  counts (COUNT):
 // cost-window taps.  Three resident CTAs per SM (80 registers, no spills): 14% faster than
 // four at 64 registers with spills, the compiler's choice without a minimum.
+//
+// A candidate at distance A from the pull's target is taken when cost + A < B, B the current state's
+// cost and distance.  Not counting, it is evaluated only if B - A > 0 (no cost is negative), only until its cost has
+// passed B - A, and not if it is the current flow bit for bit whose cost is known (known: the states' costs are
+// their flows'; a thread beyond the image starts from another pixel's state).  Counting passes evaluate every
+// candidate as the source does.
 template <bool COUNT>
 __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, float4* __restrict__ pout,
                                                const float4* __restrict__ in, const float4* __restrict__ pin, Frames F,
-                                               float flowmax, int iter, unsigned long long* counts)
+                                               float flowmax, int iter, int known, unsigned long long* counts)
 {
+    __shared__ WarpScratch<> ws[COUNT ? 1 : G * G / 32];
     __shared__ float4 buf[BUF][BUF];
     __shared__ float4 bufp[PB][PB];
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -201,9 +360,22 @@ __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, floa
     float4 ret = buf[ty + OFF][tx + OFF];
     const float curx = ret.x + (lambda0 / tau) * divx, cury = ret.y + (lambda0 / tau) * divy;
     const float lam = iter < 5 ? 0.0f : 1.0f / (2.0f * lambda0 * 5.0f);
-    auto test = [&](float nx, float ny, float cost) {
+    const int lane = (ty * G + tx) & 31;
+    const bool trust = known && x < W && y < H;
+    auto test = [&](float nx, float ny) {   // every thread of the group calls
         const float an = nx - curx, bn = ny - cury, ar = ret.x - curx, br = ret.y - cury;
-        if (cost + lam * (an * an + bn * bn) < ret.z + lam * (ar * ar + br * br)) {
+        const float A = lam * (an * an + bn * bn), B = ret.z + lam * (ar * ar + br * br);
+        float cost;
+        if (COUNT) {
+            cost = eval<true>(F, x, y, nx, ny, taps);
+        } else {
+            const float most = B - A;
+            const bool same = __float_as_uint(nx) == __float_as_uint(ret.x) && __float_as_uint(ny) == __float_as_uint(ret.y);
+            const bool need = most > 0.0f && fin(nx) && fin(ny) && !(trust && same);
+            cost = eval_warp(F, ws[(ty * G + tx) >> 5], lane, need, x, y, nx, ny, most);
+            if (!need) cost = __int_as_float(0x7f800000);
+        }
+        if (cost + A < B) {
             ret.x = nx;
             ret.y = ny;
             ret.z = cost;
@@ -211,11 +383,11 @@ __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, floa
     };
     Rng g;
     g.init_skip(skip(y * W + x, 2 * 2 * iter));
-    test(curx, cury, eval<COUNT>(F, x, y, curx, cury, taps));
+    test(curx, cury);
 #pragma unroll 1
     for (int k = 0; k < 2; k++) {   // random tries (:637-645)
         const float2 n = state_init(g, flowmax);
-        test(n.x, n.y, eval<COUNT>(F, x, y, n.x, n.y, taps));
+        test(n.x, n.y);
     }
 #pragma unroll 1
     for (int k = 0; k < 2; k++) {   // random neighbours within 5 px (:648-656)
@@ -224,7 +396,7 @@ __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, floa
         const float ry = g.next();
         const int oy = (int)((ry - 0.5f) * 2.0f * 5.0f + 0.5f);
         const float4 n = __ldg(in + (size_t)min(max(y + oy, 0), H - 1) * W + min(max(x + ox, 0), W - 1));
-        test(n.x, n.y, eval<COUNT>(F, x, y, n.x, n.y, taps));
+        test(n.x, n.y);
     }
     buf[ty + OFF][tx + OFF] = ret;
     __syncthreads();
@@ -236,7 +408,7 @@ __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, floa
             const int dx = d == 0 ? step : (d == 2 ? -step : 0), dy = d == 1 ? step : (d == 3 ? -step : 0);
             const float4 n = buf[(ty + OFF + dy) % BUF][(tx + OFF + dx) % BUF];
             __syncthreads();
-            test(n.x, n.y, eval<COUNT>(F, x, y, n.x, n.y, taps));
+            test(n.x, n.y);
             buf[ty + OFF][tx + OFF] = ret;
             __syncthreads();
         }
@@ -244,7 +416,7 @@ __global__ void __launch_bounds__(G* G, 3) k_prop(float4* __restrict__ out, floa
 #pragma unroll 1
     for (int k = 0; k < 2; k++) {   // random refinement (:700-708)
         const float2 n = state_refine(g, 1.0f);
-        test(n.x, n.y, eval<COUNT>(F, x, y, n.x, n.y, taps));
+        test(n.x, n.y);
     }
     if (x < W && y < H) {
         pout[(size_t)y * W + x] = p;
@@ -275,11 +447,25 @@ void launch_init(float4* out, const Frames& F, float flowmax, cudaStream_t st)
     k_init<<<group_grid(F.W, F.H), dim3(G, G), 0, st>>>(out, F, flowmax);
 }
 
+// known: the states' costs are their flows'
 void launch_prop(float4* out, float4* pout, const float4* in, const float4* pin, const Frames& F, float flowmax, int iter,
-                 unsigned long long* counts, cudaStream_t st)
+                 int known, unsigned long long* counts, cudaStream_t st)
 {
-    if (counts) k_prop<true><<<group_grid(F.W, F.H), dim3(G, G), 0, st>>>(out, pout, in, pin, F, flowmax, iter, counts);
-    else k_prop<false><<<group_grid(F.W, F.H), dim3(G, G), 0, st>>>(out, pout, in, pin, F, flowmax, iter, nullptr);
+    const dim3 g = group_grid(F.W, F.H), b(G, G);
+    if (counts) k_prop<true><<<g, b, 0, st>>>(out, pout, in, pin, F, flowmax, iter, known, counts);
+    else k_prop<false><<<g, b, 0, st>>>(out, pout, in, pin, F, flowmax, iter, known, nullptr);
+}
+
+size_t quad_bytes(int W, int H) { return (size_t)(W + 1) * (H + 1) * sizeof(uint4); }
+
+// the planes of Frames from both images
+void launch_frames(float4* c1, float4* c2, uint4* quad, const uint8_t* img0, const uint8_t* img1, int W, int H, size_t stride,
+                   int r, cudaStream_t st)
+{
+    launch_colour(img0, stride, W, H, c1, st);
+    k_weight_sum<<<row_grid(W, H), 128, 0, st>>>(c1, W, H, r);
+    launch_colour(img1, stride, W, H, c2, st);
+    k_quad<<<row_grid(W + 1, H + 1), 128, 0, st>>>(img1, stride, W, H, quad);
 }
 
 void launch_to_flow(float2* flow, const float4* states, int W, int H, cudaStream_t st)
@@ -324,10 +510,10 @@ inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 inline bool aligned(const void* p, size_t n) { return ((uintptr_t)p % n) == 0; }
 inline size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// workspace: both colour planes, two state and two dual fields, then (host entry) both frames,
+// workspace: both colour planes, the quad plane, two state and two dual fields, then (host entry) both frames,
 // the flow, counters
 struct SLayout {
-    enum { c1, c2, s0, s1, p0, p1, img0, img1, flow, ctr, COUNT };
+    enum { c1, c2, quad, s0, s1, p0, p1, img0, img1, flow, ctr, COUNT };
     size_t off[COUNT + 1];
     size_t total() const { return off[COUNT]; }
 };
@@ -335,7 +521,8 @@ struct SLayout {
 SLayout slayout(int W, int H, size_t stride)
 {
     const size_t N = (size_t)W * H;
-    const size_t sz[SLayout::COUNT] = {16 * N, 16 * N, 16 * N, 16 * N, 16 * N, 16 * N, stride * H, stride * H, 8 * N, 16};
+    const size_t sz[SLayout::COUNT] = {16 * N, 16 * N, quad_bytes(W, H), 16 * N, 16 * N, 16 * N, 16 * N, stride * H, stride * H,
+                                        8 * N, 16};
     SLayout L;
     size_t o = 0;
     for (int k = 0; k < SLayout::COUNT; k++) {
@@ -389,15 +576,15 @@ int run_flow(pm_svpm* h, const uint8_t* img0, const uint8_t* img1, int W, int H,
     float4* p[2] = {sat<float4>(h->ws, L, SLayout::p0), sat<float4>(h->ws, L, SLayout::p1)};
     unsigned long long* ctr = sat<unsigned long long>(h->ws, L, SLayout::ctr);
     const size_t N = (size_t)W * H;
-    launch_colour(img0, stride, W, H, c1, st);
-    launch_colour(img1, stride, W, H, c2, st);
-    const Frames F = {c1, c2, W, H, r};
+    uint4* quad = sat<uint4>(h->ws, L, SLayout::quad);
+    launch_frames(c1, c2, quad, img0, img1, W, H, stride, r, st);
+    const Frames F = {c1, c2, quad, W, H, r};
     launch_init(s[1], F, flowmax, st);
     SVPM_CUDA(h, cudaMemsetAsync(p[1], 0, N * 16, st));   // clbufp2.fill(0) (SVPMFlowCL.cpp:68)
     if (h->counting) SVPM_CUDA(h, cudaMemsetAsync(ctr, 0, 8, st));
     for (int i = 0; i < iterations; i++) {
         const int swap = i & 1;
-        launch_prop(s[swap], p[swap], s[1 - swap], p[1 - swap], F, flowmax, i + 1, h->counting ? ctr : nullptr, st);
+        launch_prop(s[swap], p[swap], s[1 - swap], p[1 - swap], F, flowmax, i + 1, 1, h->counting ? ctr : nullptr, st);
     }
     const int last = 1 - (iterations & 1);
     launch_to_flow(reinterpret_cast<float2*>(flow), s[last], W, H, st);
@@ -423,10 +610,10 @@ struct SvpmScratch {
     {
         st = s;
         const size_t N = (size_t)W * H;
-        SVPM_CUDA(nullptr, cudaMallocAsync((void**)&p, 2 * N * sizeof(float4), s));
-        launch_colour(a, stride, W, H, p, s);
-        launch_colour(b, stride, W, H, p + N, s);
-        *F = Frames{p, p + N, W, H, r};
+        SVPM_CUDA(nullptr, cudaMallocAsync((void**)&p, 2 * N * sizeof(float4) + quad_bytes(W, H), s));
+        uint4* quad = reinterpret_cast<uint4*>(p + 2 * N);
+        launch_frames(p, p + N, quad, a, b, W, H, stride, r, s);
+        *F = Frames{p, p + N, quad, W, H, r};
         return PM_OK;
     }
 };
@@ -562,7 +749,7 @@ int pm_k_svpm_prop(float* out, float* pout, const float* in, const float* pin, c
     rc = sc.make(first, second, W, H, stride, r, S(stream), &F);
     if (rc) return rc;
     launch_prop(reinterpret_cast<float4*>(out), reinterpret_cast<float4*>(pout), reinterpret_cast<const float4*>(in),
-                reinterpret_cast<const float4*>(pin), F, flowmax, iter, nullptr, S(stream));
+                reinterpret_cast<const float4*>(pin), F, flowmax, iter, 0, nullptr, S(stream));
     SVPM_CUDA(nullptr, cudaGetLastError());
     return PM_OK;
 }
