@@ -284,6 +284,12 @@ __global__ void __launch_bounds__(ROF_BX* ROF_BY) k_rof_step(float4* __restrict_
 }
 
 constexpr int RF_BX = 32, RF_BY = 16, RF_NT = 256;   // k_rof_step2: output tile and threads
+// The same for images of at most RS_TILES such tiles, two per SM: a launch then lasts as long as one
+// block, whose 256 threads take each phase of a 32x16 tile in three rounds and of a 16x8 tile in one (a
+// launch of 64x48 9.6 -> 4.6 us, 320x240 11.1 -> 7.1; 512x384, 384 tiles, 13.6 -> 14.4: the wider apron
+// costs more there).  Other tiles, 64x48 / 320x240 / 512x384, us: 32x16 with 704 threads 6.4 / 9.0 / 13.9, 32x8
+// with 416 5.1 / 7.6 / 13.9, 16x16 with 384 5.2 / 7.5 / 13.7.
+constexpr int RS_BX = 16, RS_BY = 8, RS_NT = 256, RS_TILES = 296;
 
 // two primal-dual steps in one launch (temporal blocking): the block computes the first
 // step's duals over its tile grown by two columns/rows left and above and one right and
@@ -291,7 +297,7 @@ constexpr int RF_BX = 32, RF_BY = 16, RF_NT = 256;   // k_rof_step2: output tile
 // the second step on its tile.  The fields cross DRAM once per two steps instead of twice;
 // every value is formed by the same operations as in k_rof_step, so the result is the same
 // bit for bit.  first: p = q = 0 before the first of the two steps.
-template <bool HUBER>
+template <bool HUBER, int BX, int BY, int NT>
 __device__ __forceinline__ void rof_step2_tile(float4* __restrict__ unew, float4* __restrict__ pnew,
                                                float4* __restrict__ qnew, const float4* __restrict__ u,
                                                const float4* __restrict__ p, const float4* __restrict__ q,
@@ -300,19 +306,19 @@ __device__ __forceinline__ void rof_step2_tile(float4* __restrict__ unew, float4
 {
     // duals: first step over x0-2 .. x0+BX, y0-2 .. y0+BY; the second step overwrites the
     // points x0-1 .. x0+BX-1, y0-1 .. y0+BY-1 in place (each point reads only its own first-step dual)
-    __shared__ float4 sdl[RF_BY + 3][RF_BX + 3], sdh[RF_BY + 3][RF_BX + 3];
-    __shared__ float4 su[RF_BY + 2][RF_BX + 2];   // first-step primal over x0-1 .. x0+BX, y0-1 .. y0+BY (in-image points)
-    __shared__ float4 sq[RF_BY][RF_BX];           // first-step q over the tile
+    __shared__ float4 sdl[BY + 3][BX + 3], sdh[BY + 3][BX + 3];
+    __shared__ float4 su[BY + 2][BX + 2];   // first-step primal over x0-1 .. x0+BX, y0-1 .. y0+BY (in-image points)
+    __shared__ float4 sq[BY][BX];           // first-step q over the tile
     const int tid = threadIdx.x;
-    for (int i = tid; i < (RF_BX + 3) * (RF_BY + 3); i += RF_NT) {
-        const int ex = i % (RF_BX + 3), ey = i / (RF_BX + 3);
+    for (int i = tid; i < (BX + 3) * (BY + 3); i += NT) {
+        const int ex = i % (BX + 3), ey = i / (BX + 3);
         const Dual d = rof_dual<HUBER>(u, p, dt, W, H, x0 - 2 + ex, y0 - 2 + ey, first, eps);
         sdl[ey][ex] = d.lo;
         sdh[ey][ex] = d.hi;
     }
     __syncthreads();
-    for (int i = tid; i < (RF_BX + 2) * (RF_BY + 2); i += RF_NT) {
-        const int ex = i % (RF_BX + 2), ey = i / (RF_BX + 2);
+    for (int i = tid; i < (BX + 2) * (BY + 2); i += NT) {
+        const int ex = i % (BX + 2), ey = i / (BX + 2);
         const int x = x0 - 1 + ex, y = y0 - 1 + ey;
         if (x < 0 || x >= W || y < 0 || y >= H) continue;
         const Dual c = {sdl[ey + 1][ex + 1], sdh[ey + 1][ex + 1]};
@@ -322,13 +328,13 @@ __device__ __forceinline__ void rof_step2_tile(float4* __restrict__ unew, float4
         float4 un, qn;
         primal_step(u[gi], first ? f4(0, 0, 0, 0) : q[gi], img[gi], c, l, t, lam, un, qn);
         su[ey][ex] = un;
-        if (ex >= 1 && ex <= RF_BX && ey >= 1 && ey <= RF_BY) sq[ey - 1][ex - 1] = qn;
+        if (ex >= 1 && ex <= BX && ey >= 1 && ey <= BY) sq[ey - 1][ex - 1] = qn;
     }
     __syncthreads();
     // second-step duals; the clamped neighbours of a point of this range lie inside the image
     // and inside su's range
-    for (int i = tid; i < (RF_BX + 1) * (RF_BY + 1); i += RF_NT) {
-        const int ex = i % (RF_BX + 1), ey = i / (RF_BX + 1);
+    for (int i = tid; i < (BX + 1) * (BY + 1); i += NT) {
+        const int ex = i % (BX + 1), ey = i / (BX + 1);
         const int x = x0 - 1 + ex, y = y0 - 1 + ey;
         const int xc = min(max(x, 0), W - 1) - (x0 - 1), yc = min(max(y, 0), H - 1) - (y0 - 1);
         const int xp = min(max(x + 1, 0), W - 1) - (x0 - 1), yp = min(max(y + 1, 0), H - 1) - (y0 - 1);
@@ -341,8 +347,8 @@ __device__ __forceinline__ void rof_step2_tile(float4* __restrict__ unew, float4
         sdh[ey + 1][ex + 1] = d.hi;
     }
     __syncthreads();
-    for (int i = tid; i < RF_BX * RF_BY; i += RF_NT) {
-        const int ex = i % RF_BX, ey = i / RF_BX;
+    for (int i = tid; i < BX * BY; i += NT) {
+        const int ex = i % BX, ey = i / BX;
         const int x = x0 + ex, y = y0 + ey;
         if (x >= W || y >= H) continue;
         const Dual c = {sdl[ey + 2][ex + 2], sdh[ey + 2][ex + 2]};
@@ -358,15 +364,15 @@ __device__ __forceinline__ void rof_step2_tile(float4* __restrict__ unew, float4
     }
 }
 
-template <bool HUBER>
-__global__ void __launch_bounds__(RF_NT) k_rof_step2(float4* __restrict__ unew, float4* __restrict__ pnew,
+template <bool HUBER, int BX, int BY, int NT>
+__global__ void __launch_bounds__(NT) k_rof_step2(float4* __restrict__ unew, float4* __restrict__ pnew,
                                                    float4* __restrict__ qnew, const float4* __restrict__ u,
                                                    const float4* __restrict__ p, const float4* __restrict__ q,
                                                    const float4* __restrict__ img, const float4* __restrict__ dt,
                                                    float4 lam, int W, int H, int first, float eps)
 {
-    rof_step2_tile<HUBER>(unew, pnew, qnew, u, p, q, img, dt, lam, W, H, first, eps, blockIdx.x * RF_BX,
-                          blockIdx.y * RF_BY);
+    rof_step2_tile<HUBER, BX, BY, NT>(unew, pnew, qnew, u, p, q, img, dt, lam, W, H, first, eps, blockIdx.x * BX,
+                          blockIdx.y * BY);
 }
 
 static_assert(RF_BX == SMOOTH_TW && RF_BY == SMOOTH_TH16 && ROF_BX == SMOOTH_TW && ROF_BY == SMOOTH_TH8,
@@ -435,7 +441,7 @@ __global__ void __launch_bounds__(RF_NT) k_rof_step2_b(const SmoothArgs* __restr
         const uint2 job = jobs[j];
         const SmoothArgs& A = tab[job.x];
         const PdStep s = pd_step(A, launch, launches);
-        rof_step2_tile<false>(s.unew, s.pnew, s.qnew, s.u, s.p, s.q, A.tmp, A.dt, lam, A.W, A.H, launch == 0, 0.0f,
+        rof_step2_tile<false, RF_BX, RF_BY, RF_NT>(s.unew, s.pnew, s.qnew, s.u, s.p, s.q, A.tmp, A.dt, lam, A.W, A.H, launch == 0, 0.0f,
                               (int)(job.y & 0xffffu) * RF_BX, (int)(job.y >> 16) * RF_BY);
     }
 }
@@ -851,7 +857,8 @@ void launch_pd(float4* out, const float4* input, const float4* dt, float4 lam, f
     const int steps = (iters > 0 && iters % 2 == 0) ? iters : iters + 1;
     const int launches = pd_launch_count(iters);
     const dim3 b1(ROF_BX, ROF_BY), g1 = grid2d(W, H, b1);
-    const dim3 b2(RF_NT), g2((W + RF_BX - 1) / RF_BX, (H + RF_BY - 1) / RF_BY);
+    const dim3 g2((W + RF_BX - 1) / RF_BX, (H + RF_BY - 1) / RF_BY), gs((W + RS_BX - 1) / RS_BX, (H + RS_BY - 1) / RS_BY);
+    const bool small = g2.x * g2.y <= RS_TILES;
     // launch j writes `out` when (launches - 1 - j) is even, so that the last lands in `out`
     const float4* ucur = input;
     for (int j = 0; j < launches; j++) {
@@ -860,9 +867,12 @@ void launch_pd(float4* out, const float4* input, const float4* dt, float4 lam, f
         if (j == 0 && steps % 2)
             k_rof_step<HUBER><<<g1, b1, 0, st>>>(unew, p[pi], q[pi], ucur, p[1 - pi], q[1 - pi], input, dt, lam, W, H,
                                                  1, eps);
+        else if (small)
+            k_rof_step2<HUBER, RS_BX, RS_BY, RS_NT><<<gs, RS_NT, 0, st>>>(unew, p[pi], q[pi], ucur, p[1 - pi], q[1 - pi],
+                                                                          input, dt, lam, W, H, j == 0, eps);
         else
-            k_rof_step2<HUBER><<<g2, b2, 0, st>>>(unew, p[pi], q[pi], ucur, p[1 - pi], q[1 - pi], input, dt, lam, W,
-                                                  H, j == 0, eps);
+            k_rof_step2<HUBER, RF_BX, RF_BY, RF_NT><<<g2, RF_NT, 0, st>>>(unew, p[pi], q[pi], ucur, p[1 - pi], q[1 - pi],
+                                                                          input, dt, lam, W, H, j == 0, eps);
         ucur = unew;
     }
 }

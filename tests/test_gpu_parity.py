@@ -601,6 +601,29 @@ def test_primal_dual_steps_ragged_sizes(D, orc, W, H):
         assert bits_equal(host(o), orc.huber(inp, dt, lam, 1e-4, iters)).all(), ("huber", iters)
 
 
+@pytest.mark.parametrize("W,H", [(577, 256), (593, 257)])
+def test_primal_dual_steps_both_tiles(D, orc, W, H):
+    """The largest image of the small smoothing tile (296 tiles of 32x16 or fewer: 19 x 16 = 304 is past it, as
+    is 19 x 17) and ragged edges of the large one, on finite fields"""
+    for w, h in ((W, H), (W - 32, H - 16)):
+        rng = np.random.default_rng(w * 131 + h)
+        inp = rng.standard_normal((h, w, 4)).astype(np.float32)
+        dt = rng.uniform(-1.0, 1.0, (h, w, 4)).astype(np.float32)
+        di, dd = dev(D.t, inp), dev(D.t, dt)
+        scratch = D.t.zeros(D.L.pm_rof_scratch_bytes(w, h), dtype=D.t.uint8, device="cuda")
+        lam = [1.7, 0.9, 2.3, 1.1]
+        lam_c = (C.c_float * 4)(*lam)
+        for iters in (2, 5):
+            o = D.f4(h, w)
+            assert D.L.pm_k_rof(o.data_ptr(), di.data_ptr(), dd.data_ptr(), lam_c, iters, w, h, scratch.data_ptr(),
+                                stream(D.t)) == 0
+            assert bits_equal(host(o), orc.rof(inp, dt, lam, iters)).all(), ("rof", w, h, iters)
+            o = D.f4(h, w)
+            assert D.L.pm_k_huber(o.data_ptr(), di.data_ptr(), dd.data_ptr(), lam_c, 1e-4, iters, w, h,
+                                  scratch.data_ptr(), stream(D.t)) == 0
+            assert bits_equal(host(o), orc.huber(inp, dt, lam, 1e-4, iters)).all(), ("huber", w, h, iters)
+
+
 @pytest.mark.parametrize("case", depth_cases())
 def test_depth_pipeline_strict_matches_reference_golden(native, torch_cuda, case):
     from cvt_b200 import PMHuberStereo
