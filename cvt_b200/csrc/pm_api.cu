@@ -362,6 +362,7 @@ PropParams prop_params(const pm_handle* h, const LevelBufs& B, int view, int ite
     P.tmp_self = B.pself;
     P.tmp_nb = B.pnb;
     P.dual = 0;
+    P.known = 1;
     return P;
 }
 
@@ -558,6 +559,7 @@ int run_depth(pm_handle* h, void* ws, const uint8_t* left, const uint8_t* right,
         P.tmp_self = at<float4>(ws, L, Layout::pself);
         P.tmp_nb = at<float4>(ws, L, Layout::pnb);
         P.dual = 0;
+        P.known = 1;
         launch_propagate(P, F, st);   // :263-264
         if (views == 2) {
             P.V = VR;
@@ -1717,6 +1719,7 @@ int pm_k_propagate(float* out, const float* old, const float* bw1, const float* 
     P.smooth = (const float4*)smooth;
     P.theta = theta;
     P.dmax = dmax;
+    P.known = 0;
     P.lr = lr;
     P.iter = iter;
     P.vin_count = vin_count;

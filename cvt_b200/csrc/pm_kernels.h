@@ -37,6 +37,7 @@ struct PropParams {
     float4* tmp_self;               // per-pixel state between the three propagate kernels
     float4* tmp_nb;
     int dual;                       // the window-loop kernels run as two variants (pm_window.cuh)
+    int known;                      // the costs in `old` are those of its planes (k_prop_chain)
     int owners;                     // pixels per warp row of the propagate kernels (set by the launchers)
 };
 

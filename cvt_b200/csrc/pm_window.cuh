@@ -516,7 +516,7 @@ __device__ __forceinline__ int pair_mismatch(const PairSigns& d, uint32_t sb1)
 // the largest half so far, each with its bit 15 set: 0xffff when some sign was unsure
 __device__ __forceinline__ uint32_t unsure_max(uint32_t m, const PairSigns& d)
 {
-    return __vmaxu2(m, __vmaxu2(d.yw | 0x80008000u, d.xz | 0x80008000u));
+    return __vimax3_u16x2(m, d.yw | 0x80008000u, d.xz | 0x80008000u);
 }
 __device__ __forceinline__ bool unsure(uint32_t m) { return (m >> 16) == 0xffffu || (m & 0xffffu) == 0xffffu; }
 
