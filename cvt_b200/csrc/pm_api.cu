@@ -207,12 +207,13 @@ int prof_collect(pm_handle* h, cudaStream_t st)
 struct Layout {
     enum {
         Lbw, Rbw, Lg, Rg, LDT, RDT, Ls, Rs, tmp, mL0, mL1, mR0, mR1, chk, nrm,   // float4 x N
-        pself, pnb,                                                             // float4 x N
+        pself, pnb, pselfR, pnbR,                                               // float4 x N (left, right view)
+        klist,                                                                  // int x N
         vb1c, vb2c,                                                             // int x N
         vb1s, vb2s,                                                             // u64 x N
         texL, texR,                                                             // texel rows
         rof,                                                                    // rof scratch
-        ctr, errf,                                                              // counters (4 u64), error int
+        ctr, errf, kcount,                                                      // counters (4 u64), error int, list length
         img0, img1, disp, dmap, nmap, initd, initn,                             // staging for host entry
         initdR, initnR,                                                         // right-view init (pyramid)
         outpL, outpR,                                                           // plane outputs for host entry
@@ -236,11 +237,15 @@ Layout layout(int W, int H, size_t stride)
     put(Layout::vb2s, L.N * 8);
     put(Layout::pself, L.N * 16);
     put(Layout::pnb, L.N * 16);
+    put(Layout::pselfR, L.N * 16);
+    put(Layout::pnbR, L.N * 16);
+    put(Layout::klist, L.N * 4);
     put(Layout::texL, tex_bytes(W, H));
     put(Layout::texR, tex_bytes(W, H));
     put(Layout::rof, rof_scratch_bytes(W, H));
     put(Layout::ctr, 64);
     put(Layout::errf, 64);
+    put(Layout::kcount, 64);
     put(Layout::img0, stride * H);
     put(Layout::img1, stride * H);
     put(Layout::disp, L.N * 4);
@@ -283,7 +288,8 @@ struct LevelBufs {
     int *vb1c, *vb2c;
     unsigned long long *vb1s, *vb2s;
     void* rofs;
-    float4 *texL, *texR, *pself, *pnb;
+    float4 *texL, *texR, *pself[2], *pnb[2];   // [view]
+    int *klist, *kcount;
     ViewData VL, VR;
     int W, H;
 };
@@ -311,8 +317,12 @@ LevelBufs level_bufs(void* ws, const Layout& L, int W, int H, int r)
     B.rofs = at<void>(ws, L, Layout::rof);
     B.texL = at<float4>(ws, L, Layout::texL);
     B.texR = at<float4>(ws, L, Layout::texR);
-    B.pself = at<float4>(ws, L, Layout::pself);
-    B.pnb = at<float4>(ws, L, Layout::pnb);
+    B.pself[0] = at<float4>(ws, L, Layout::pself);
+    B.pnb[0] = at<float4>(ws, L, Layout::pnb);
+    B.pself[1] = at<float4>(ws, L, Layout::pselfR);
+    B.pnb[1] = at<float4>(ws, L, Layout::pnbR);
+    B.klist = at<int>(ws, L, Layout::klist);
+    B.kcount = at<int>(ws, L, Layout::kcount);
     B.VL = make_view(B.texL, B.texR, W, H, r);
     B.VR = make_view(B.texR, B.texL, W, H, r);
     B.W = W;
@@ -359,8 +369,10 @@ PropParams prop_params(const pm_handle* h, const LevelBufs& B, int view, int ite
     }
     P.counters = h->counting ? ctr : nullptr;
     P.error = errf;
-    P.tmp_self = B.pself;
-    P.tmp_nb = B.pnb;
+    P.tmp_self = B.pself[view];
+    P.tmp_nb = B.pnb[view];
+    P.list = B.klist;
+    P.list_count = B.kcount;
     P.dual = 0;
     P.known = 1;
     return P;
@@ -383,6 +395,7 @@ int level_begin(pm_handle* h, const LevelBufs& B, const uint8_t* left, const uin
     if (views == 2) launch_prep(right, stride, W, H, r, F, B.Rbw, B.Rg, B.RDT, st);
     else launch_prep(right, stride, W, H, r, F, B.Rbw, B.Rg, nullptr, st);
     // clear the smoothing images (:457-458) and both view buffers (:487)
+    PM_CUDA(h, cudaMemsetAsync(B.kcount, 0, 64, st));
     PM_CUDA(h, cudaMemsetAsync(B.Ls, 0, N * 16, st));
     PM_CUDA(h, cudaMemsetAsync(B.Rs, 0, N * 16, st));
     launch_view_clear(B.vb1c, B.vb1s, N, st);
@@ -503,6 +516,7 @@ int run_depth(pm_handle* h, void* ws, const uint8_t* left, const uint8_t* right,
     int* errf = at<int>(ws, L, Layout::errf);
 
     PM_CUDA(h, cudaMemsetAsync(ctr, 0, 64, st));
+    PM_CUDA(h, cudaMemsetAsync(at<int>(ws, L, Layout::kcount), 0, 64, st));
     PM_CUDA(h, cudaMemsetAsync(errf, 0, 64, st));
     h->ev_used = 0;
     prof_mark(h, st, PM_PHASE_PREP, 0);
@@ -558,10 +572,14 @@ int run_depth(pm_handle* h, void* ws, const uint8_t* left, const uint8_t* right,
         P.error = errf;
         P.tmp_self = at<float4>(ws, L, Layout::pself);
         P.tmp_nb = at<float4>(ws, L, Layout::pnb);
+        P.list = at<int>(ws, L, Layout::klist);
+        P.list_count = at<int>(ws, L, Layout::kcount);
         P.dual = 0;
         P.known = 1;
         launch_propagate(P, F, st);   // :263-264
         if (views == 2) {
+            P.tmp_self = at<float4>(ws, L, Layout::pselfR);
+            P.tmp_nb = at<float4>(ws, L, Layout::pnbR);
             P.V = VR;
             P.out = mR[1 - swap];
             P.old = mR[swap];
@@ -1731,6 +1749,8 @@ int pm_k_propagate(float* out, const float* old, const float* bw1, const float* 
     P.error = d_err;
     float4* tmp = nullptr;
     PM_CUDA(nullptr, cudaMallocAsync((void**)&tmp, (size_t)W * H * 2 * sizeof(float4), S(stream)));
+    P.list = nullptr;
+    P.list_count = nullptr;
     P.tmp_self = tmp;
     P.tmp_nb = tmp + (size_t)W * H;
     launch_propagate(P, fused, S(stream));

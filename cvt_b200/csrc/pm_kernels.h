@@ -34,8 +34,12 @@ struct PropParams {
     unsigned long long* vout_src;
     unsigned long long* counters;   // null: not counted
     int* error;                     // incremented if a view-buffer insert gave up
-    float4* tmp_self;               // per-pixel state between the three propagate kernels
+    // per-pixel state between the three propagate kernels: the plane after the candidates and its Gauss-Newton
+    // result; with `list` they are this view's own and still hold the previous iteration's
+    float4* tmp_self;
     float4* tmp_nb;
+    int* list;                      // may be null: pixels whose Gauss-Newton steps are to be run, and their
+    int* list_count;                // number (0 between passes)
     int dual;                       // the window-loop kernels run as two variants (pm_window.cuh)
     int known;                      // the costs in `old` are those of its planes (k_prop_chain)
     int owners;                     // pixels per warp row of the propagate kernels (set by the launchers)
@@ -67,7 +71,7 @@ void prop_tile_shape(int* w, int* h);
 // false for any other width
 bool prop_batch_tile_shape(int tile_w, int* w, int* h);
 // pairs per batched propagate launch: their arguments are one kernel parameter block
-// (128 x 192 bytes, within the 32,764 bytes a launch may pass)
+// (128 x 208 bytes, within the 32,764 bytes a launch may pass)
 constexpr int PROP_GROUP = 128;
 struct PropGroup {
     PropParams p[PROP_GROUP];

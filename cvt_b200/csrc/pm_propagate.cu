@@ -189,6 +189,23 @@ __device__ __forceinline__ void chain_tile(const PropParams& P, WarpScratch<>* w
             sd_self = sd;
         }
     }
+    // Within a run the Gauss-Newton steps of a plane that the pixel already had after the previous iteration's
+    // candidates would give the result that still lies in tmp_nb.  The others are listed, a warp's pixels
+    // together (launch_pass; the list's order changes nothing, each pixel is on its own).
+    if (!GEN && P.list) {
+        bool todo = own;
+        if (own && P.iter > 0) {
+            const float4 was = P.tmp_self[idx];
+            todo = __float_as_uint(was.x) != __float_as_uint(self.x) || __float_as_uint(was.y) != __float_as_uint(self.y) ||
+                   __float_as_uint(was.z) != __float_as_uint(self.z);
+        }
+        const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
+        const unsigned m = __ballot_sync(0xffffffffu, todo);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(P.list_count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (todo) P.list[at + __popc(m & ((1u << lane) - 1u))] = (int)idx;
+    }
     if (own) P.tmp_self[idx] = self;
 }
 
@@ -223,6 +240,20 @@ __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt(PropPa
     Counters cnt = {0, 0, 0, 0};
     klt_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
+}
+
+// the same for the pixels of P.list
+template <bool F>
+__global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt_list(PropParams P)
+{
+    if (variant_skips<false>(P.V, P.dual)) return;
+    const int i = blockIdx.x * PROP_THREADS + threadIdx.x;
+    if (i >= *P.list_count) return;
+    const int idx = P.list[i];
+    const int py = idx / P.V.W, px = idx - py * P.V.W;
+    float4 nb = P.tmp_self[idx];
+    for (int k = 0; k < 6; k++) nb = klt2_pair<F>(P.V, px, py, nb);
+    P.tmp_nb[idx] = nb;
 }
 
 // the same with P.owners <= WARP_KLT pixels per warp (prop_owners)
@@ -291,6 +322,7 @@ __global__ void __launch_bounds__(PROP_THREADS) k_prop_final(PropParams P)
     if (variant_skips<GEN>(P.V, P.dual)) return;
     __shared__ WarpScratch<> ws[GEN ? 1 : PROP_THREADS / 32];
     Counters cnt = {0, 0, 0, 0};
+    if (!GEN && P.list && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *P.list_count = 0;
     final_tile<F, COUNT, GEN>(P, ws, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
@@ -416,6 +448,7 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
     for (int i = 0; i < n; i++) {
         tab.p[i] = group[i];
         tab.p[i].owners = tile_w;
+        tab.p[i].list = nullptr;   // the batched Gauss-Newton kernels run every pixel
     }
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
@@ -465,6 +498,7 @@ void launch_pass(const PropParams& Q, cudaStream_t st)
     k_prop_chain<F, false, false><<<g, b, 0, st>>>(Q);
     k_prop_chain<F, false, true><<<gg, b, 0, st>>>(G);
     if (Q.owners <= WARP_KLT) k_prop_klt_warp<F><<<g, b, 0, st>>>(Q);
+    else if (Q.list) k_prop_klt_list<F><<<(Q.V.W * Q.V.H + PROP_THREADS - 1) / PROP_THREADS, PROP_THREADS, 0, st>>>(Q);
     else k_prop_klt<F, false, false><<<gg, b, 0, st>>>(G);
     k_prop_klt<F, false, true><<<gg, b, 0, st>>>(G);
     k_prop_final<F, false, false><<<g, b, 0, st>>>(Q);
@@ -495,6 +529,7 @@ void launch_propagate(const PropParams& P, int fused, cudaStream_t st)
     } else {
         Q.dual = 1;
         Q.owners = prop_owners(P.V.W, P.V.H);
+        if (Q.owners <= WARP_KLT) Q.list = nullptr;
         if (fused) launch_pass<true>(Q, st);
         else launch_pass<false>(Q, st);
     }
