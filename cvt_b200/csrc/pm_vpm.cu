@@ -16,7 +16,8 @@
 // A pass is three kernels, as the main path's (candidates, Gauss-Newton steps, their evaluation), over the
 // pair-plane loops of pm_window.cuh / pm_warp.cuh.  The general loops below, one kernel per pass, count the
 // taps (pm_vpm_set_counting) and serve injected gradients that are not finite.  Measured at 640x480, r = 10,
-// 8 iterations: general loops 95.7 ms a call, the three kernels 56.7 (30.2 + 21.9 + 3.6).
+// 8 iterations: general loops 95.7 ms a call, the three kernels 50.1 (30.1 + 15.9 + 3.1; 56.7 with the
+// Gauss-Newton steps of every pixel in every pass).
 //
 // Arithmetic is the reference's FP32 sequence (the file is compiled with -fmad=false): every
 // result equals the restatement in oracle/pm_oracle.cpp bit for bit.  The one double in the
@@ -328,8 +329,13 @@ struct VPixel {
 // neighbour states.  A candidate whose plane is the current one's bit for bit has its cost and cannot be below
 // it; it is skipped when the states' costs are their planes' (known; not for states from outside).
 // Bound by instruction issue, as the main path's candidate kernel; 5 blocks per SM = 96 registers.
+//
+// Within a run a plane that the candidates left as they did in the previous iteration (prev) went through the
+// Gauss-Newton steps then and beat their result; nothing is left to do for it.  The other pixels are listed
+// for k_steps and k_settle (list[0] their number, list[1..] the pixels; a warp's together).
 __global__ void __launch_bounds__(PT, 5) k_cand(float4* __restrict__ cur_out, const float4* __restrict__ in, Views V,
-                                             float dmax, int iter, int owners, int known)
+                                             float dmax, int iter, int owners, int known, float4* __restrict__ prev,
+                                             int* __restrict__ list)
 {
     if (variant_skips<false>(V, 1)) return;
     __shared__ WarpScratch<VPM> ws[PT / 32];
@@ -352,7 +358,52 @@ __global__ void __launch_bounds__(PT, 5) k_cand(float4* __restrict__ cur_out, co
         s.w = patch_eval_warp<false, true, VPM>(V, ws[threadIdx.y], P.lane, need, P.x, P.y, s, cur.w);
         if (need && s.w < cur.w) cur = s;
     }
+    if (list) {
+        bool todo = P.own;
+        if (P.own && iter > 0) {
+            const float4 was = prev[P.i];
+            todo = __float_as_uint(was.x) != __float_as_uint(cur.x) || __float_as_uint(was.y) != __float_as_uint(cur.y) ||
+                   __float_as_uint(was.z) != __float_as_uint(cur.z);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, todo);
+        int at = 0;
+        if (P.lane == 0 && m) at = atomicAdd(list, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (todo) {
+            list[1 + at + __popc(m & ((1u << P.lane) - 1u))] = (int)P.i;
+            prev[P.i] = cur;
+        }
+    }
     if (P.own) cur_out[P.i] = cur;
+}
+
+// three Gauss-Newton steps (:347-349) of the listed pixels
+__global__ void __launch_bounds__(PT, 5) k_steps_list(float4* __restrict__ out, const float4* __restrict__ cur, Views V,
+                                                   const int* __restrict__ list)
+{
+    if (variant_skips<false>(V, 1)) return;
+    const int i = blockIdx.x * PT + threadIdx.x;
+    if (i >= list[0]) return;
+    const int idx = list[1 + i], y = idx / V.W;
+    float4 s = __ldg(cur + idx);
+#pragma unroll 1
+    for (int k = 0; k < 3; k++) s = klt2_pair<false, VPM>(V, idx - y * V.W, y, s);
+    out[idx] = s;
+}
+
+// the evaluation of their result (:350-358), as k_settle
+__global__ void __launch_bounds__(PT, 5) k_settle_list(float4* __restrict__ out, const float4* __restrict__ steps, Views V,
+                                                    const int* __restrict__ list)
+{
+    if (variant_skips<false>(V, 1)) return;
+    __shared__ WarpScratch<VPM> ws[PT / 32];
+    const int i = blockIdx.x * PT + threadIdx.x, n = list[0];
+    if ((i & ~31) >= n) return;   // a whole warp
+    const bool own = i < n;
+    const int idx = own ? list[1 + i] : 0, y = idx / V.W, x = idx - y * V.W;
+    float4 cur = own ? out[idx] : f4(0.0f, 0.0f, 0.0f, 0.0f), s = own ? __ldg(steps + idx) : cur;
+    s.w = patch_eval_warp<false, false, VPM>(V, ws[threadIdx.x >> 5], threadIdx.x & 31, own, x, y, s, cur.w);
+    if (own && s.w < cur.w) out[idx] = s;
 }
 
 // three Gauss-Newton steps (:347-349), a thread per pixel or, on small images, a few pixels per warp
@@ -422,9 +473,10 @@ void launch_init(float4* out, const Views& V, float dmax, const float* initdisp,
     k_init<<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, V, dmax, initdisp);
 }
 
-// one pass from `in` to `out`; steps: a W*H field; known: every state's cost is its plane's
+// one pass from `in` to `out`; steps: a W*H field.  known: a run, every state's cost is its plane's; prev
+// and list (W*H planes, W*H + 1 ints) then hold what k_cand keeps from one iteration to the next
 void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, float dmax, int iter, int known,
-                 unsigned long long* counts, cudaStream_t st)
+                 float4* prev, int* list, unsigned long long* counts, cudaStream_t st)
 {
     if (counts) {
         k_iter<true><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, counts);
@@ -432,10 +484,18 @@ void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, f
     }
     const int owners = prop_owners(V.W, V.H);
     const dim3 b(32, PT / 32), g((V.W + owners - 1) / owners, (V.H + PT / 32 - 1) / (PT / 32));
-    k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known);
-    if (owners <= WARP_KLT) k_steps<true><<<g, b, 0, st>>>(steps, out, V, owners);
-    else k_steps<false><<<g, b, 0, st>>>(steps, out, V, owners);
-    k_settle<<<g, b, 0, st>>>(out, steps, V, owners);
+    if (known && owners > WARP_KLT) {
+        const int blocks = (int)(((size_t)V.W * V.H + PT - 1) / PT);
+        cudaMemsetAsync(list, 0, sizeof(int), st);
+        k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known, prev, list);
+        k_steps_list<<<blocks, PT, 0, st>>>(steps, out, V, list);
+        k_settle_list<<<blocks, PT, 0, st>>>(out, steps, V, list);
+    } else {
+        k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known, nullptr, nullptr);
+        if (owners <= WARP_KLT) k_steps<true><<<g, b, 0, st>>>(steps, out, V, owners);
+        else k_steps<false><<<g, b, 0, st>>>(steps, out, V, owners);
+        k_settle<<<g, b, 0, st>>>(out, steps, V, owners);
+    }
     k_iter<false><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, nullptr);
 }
 
@@ -485,10 +545,11 @@ inline cudaStream_t S(void* s) { return static_cast<cudaStream_t>(s); }
 inline bool aligned(const void* p, size_t n) { return ((uintptr_t)p % n) == 0; }
 inline size_t up256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// workspace: texel planes of both images, two state fields, the Gauss-Newton results, then (host
+// workspace: texel planes of both images, two state fields, the Gauss-Newton results, the
+// planes of the previous iteration's candidates and the list of changed pixels, then (host
 // entry) both images, the initial disparities, the disparities, counters
 struct VLayout {
-    enum { tex0, tex1, s0, s1, steps, img0, img1, initd, disp, ctr, COUNT };
+    enum { tex0, tex1, s0, s1, steps, prev, list, img0, img1, initd, disp, ctr, COUNT };
     size_t off[COUNT + 1];
     size_t total() const { return off[COUNT]; }
 };
@@ -496,8 +557,8 @@ struct VLayout {
 VLayout vlayout(int W, int H, size_t stride)
 {
     const size_t N = (size_t)W * H;
-    const size_t sz[VLayout::COUNT] = {tex_bytes(W, H), tex_bytes(W, H), 16 * N, 16 * N, 16 * N, stride * H, stride * H,
-                                        4 * N, 4 * N, 16};
+    const size_t sz[VLayout::COUNT] = {tex_bytes(W, H), tex_bytes(W, H), 16 * N, 16 * N, 16 * N, 16 * N, 4 * (N + 1), stride * H,
+                                        stride * H, 4 * N, 4 * N, 16};
     VLayout L;
     size_t o = 0;
     for (int k = 0; k < VLayout::COUNT; k++) {
@@ -554,7 +615,8 @@ int run_simple(pm_vpm* h, const uint8_t* img0, const uint8_t* img1, int W, int H
     if (h->counting) VPM_CUDA(h, cudaMemsetAsync(ctr, 0, 16, st));
     int swap = 0;
     for (int i = 0; i < h->iterations; i++) {
-        launch_iter(s[swap], s[1 - swap], steps, V, h->dmax, i, 1, h->counting ? ctr : nullptr, st);
+        launch_iter(s[swap], s[1 - swap], steps, V, h->dmax, i, 1, vat<float4>(h->ws, L, VLayout::prev),
+                    vat<int>(h->ws, L, VLayout::list), h->counting ? ctr : nullptr, st);
         swap = 1 - swap;
     }
     launch_disparity(disp, s[1 - swap], W, H, 1.0f, st);
@@ -739,7 +801,7 @@ int pm_k_vpm_iter(float* out, const float* in, const uint8_t* c1, const float* g
     rc = sc.make(c1, g1, c2, g2, W, H, stride, r, S(stream), &V);
     if (rc) return rc;
     launch_iter(reinterpret_cast<float4*>(out), reinterpret_cast<const float4*>(in), sc.steps, V, dmax, iter, 0, nullptr,
-                S(stream));
+                nullptr, nullptr, S(stream));
     VPM_CUDA(nullptr, cudaGetLastError());
     return PM_OK;
 }
