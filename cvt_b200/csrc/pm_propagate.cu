@@ -1,7 +1,8 @@
 // pmhstereo_propagate_view (cvt/cl/kernel/pmhstereo.cl:880-1071) on sm_100a, as three
 // kernels over the same pixels:
 //   k_prop_chain  the candidate chain up to the randomized refinement (:927-1028)
-//   k_prop_klt    the six Gauss-Newton steps (:1034-1038)
+//   k_prop_klt    the six Gauss-Newton steps (:1034-1038); k_prop_klt_list runs them for listed pixels,
+//                 k_prop_klt_warp with few pixels per warp
 //   k_prop_final  the evaluation of their result, the view scatter and the output (:1039-1070)
 // The state between them is `self` and the Gauss-Newton result (two float4 fields).
 //
