@@ -198,7 +198,7 @@ __device__ __forceinline__ float expf_neg(float x)
     p = fmaf(p, r, 1.0f);
     p = fmaf(p, r, 1.0f);
     // p 2^n by adding n to p's exponent field: the bits of t are those of M plus n, and the bits of M
-    // vanish in the shift
+    // vanish in the shift.  Not a NaN for a NaN x: arguments outside the range take expf_
     return __int_as_float(__float_as_int(p) + (__float_as_int(t) << 23));
 }
 
@@ -208,6 +208,13 @@ template <bool F>
 __device__ __forceinline__ float support_weight(float dx, float dy, float dz)
 {
     return expf_neg(-fabsf(gray_dot<F>(dx, dy, dz)) * 12.0f);
+}
+
+// the same for injected colours of any value, NaN and infinities included
+template <bool F>
+__device__ __forceinline__ float support_weight_any(float dx, float dy, float dz)
+{
+    return expf_(-fabsf(gray_dot<F>(dx, dy, dz)) * 12.0f);
 }
 
 // SAMPLER_BILINEAR (:71) read at (u, row + 0.5): OpenCL 1.2 s8.2 with the vertical

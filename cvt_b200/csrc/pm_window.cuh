@@ -252,7 +252,7 @@ __device__ __forceinline__ bool eval_sample(const float4* __restrict__ q1, const
     const float p2x = F ? fmaf(s.x, qx, byq) + s.z : s.x * qx + byq + s.z;
     if (p2x < 0 || p2x >= fW) return false;
     const float4 q = __ldg(q1);   // compact texel
-    const float w = support_weight<F>(q.x - in.x, q.y - in.y, q.z - in.z);
+    const float w = support_weight_any<F>(q.x - in.x, q.y - in.y, q.z - in.z);
     const float t = (p2x + 0.5f) - 0.5f;
     Texel tx;
     if (fin(t)) {
@@ -346,7 +346,7 @@ __device__ __forceinline__ float4 klt2_general(const ViewData& V, int px, int py
         for (int n = dx1 - dx0; n >= 0; n--, q1++, qx += 1.0f) {
             const float4 q = __ldg(q1);   // compact texel
             const float4 val1 = make_float4(q.x - c1.x, q.y - c1.y, q.z - c1.z, 0.0f);
-            const float w1 = support_weight<F>(val1.x, val1.y, val1.z);
+            const float w1 = support_weight_any<F>(val1.x, val1.y, val1.z);
             const uint32_t sb1 = __float_as_uint(q.w);
             const KltWeights kw = klt_weights<F>(w1);
             const float p2x = F ? fmaf(s.x, qx, byq) + s.z : s.x * qx + byq + s.z;

@@ -200,6 +200,36 @@ def test_tiny_colours_take_exact_division(D, orc):
         assert bits_equal(init, orc.init(bwL, bwR, gL, gR, r, dmax, 1, fused=f)).all()
 
 
+def test_colours_of_any_value_match_oracle(D, orc):
+    """Injected colours far outside [0, 1]: NaN, infinities, and finite ones whose support weights are
+    denormal or 0 (exp of arguments below -87).  Costs, Gauss-Newton steps, init and a propagate pass equal
+    the oracle's (a NaN equals any NaN)."""
+    g = load_golden("lr_40x28")
+    W, H, r, dmax, iters, pp, views = spec_of(g)
+    gL, gR, P = g["gL"], g["gR"], g["k_planes"]
+    dgL, dgR, dP = (dev(D.t, a) for a in (gL, gR, P))
+    sm = np.zeros((H, W, 4), np.float32)
+    values = np.array([np.nan, np.inf, -np.inf, 1e30, -3e38, 7.27, 7.3, 8.0, -8.6, 8.7, 100.0], np.float32)
+    rng = np.random.default_rng(3)
+    for k, some in enumerate((values[:1], values[5:10], values)):
+        bwL, bwR = g["bwL"].copy(), g["bwR"].copy()
+        for bw in (bwL, bwR):
+            at = rng.random((H, W, 3)) < 0.03
+            bw[..., :3][at] = rng.choice(some, int(at.sum()))
+        dL, dR = dev(D.t, bwL), dev(D.t, bwR)
+        for f in (0, 1):
+            for m in (1e10, 0.2):
+                assert bits_equal(host(D.cost(dP, dL, dR, dgL, dgR, r, m, f)),
+                                  orc.cost(P, bwL, bwR, gL, gR, r, m, fused=f)).all(), (k, f, m)
+            assert bits_equal(host(D.klt(dP, dL, dR, dgL, dgR, r, f)),
+                              orc.klt(P, bwL, bwR, gL, gR, r, fused=f)).all(), (k, f)
+            init = host(D.init(dL, dR, dgL, dgR, r, dmax, 1, f))
+            assert bits_equal(init, orc.init(bwL, bwR, gL, gR, r, dmax, 1, fused=f)).all(), (k, f)
+            want = orc.propagate(P, bwL, bwR, gL, gR, sm, 0.3, r, dmax, 1, 1, fused=f)[0]
+            got = D.propagate(dP, dL, dR, dgL, dgR, dev(D.t, sm), 0.3, r, dmax, 1, 1, fused=f)
+            assert bits_equal(host(got), want).all(), (k, f)
+
+
 def pair_planes(rng, W, H, grad2):
     """planes that meet the window loops' special cases: matched columns around both image borders, around
     powers of two and at whole columns, tap weights at a sign change of the interpolated gradient, steep
