@@ -203,11 +203,14 @@ int prof_collect(pm_handle* h, cudaStream_t st)
     return PM_OK;
 }
 
-// workspace layout for a W x H pair (float4 fields unless noted)
+// workspace layout for a W x H pair (float4 fields unless noted).  Fields that are dead when another is written
+// share its place: the texel planes hold all that the passes read of bw and grad, so the per-view state
+// between the propagate kernels lies there; the LR result takes the smoothing input's place after
+// the last pass; and normals derived from a given disparity are read by init, before mL1 is written.
 struct Layout {
     enum {
-        Lbw, Rbw, Lg, Rg, LDT, RDT, Ls, Rs, tmp, mL0, mL1, mR0, mR1, chk, nrm,   // float4 x N
-        pself, pnb, pselfR, pnbR,                                               // float4 x N (left, right view)
+        Lbw, Rbw, Lg, Rg, LDT, RDT, Ls, Rs, tmp, mL0, mL1, mR0, mR1,             // float4 x N
+        chk, nrm, pself, pnb, pselfR, pnbR,                                     // in tmp, mL1, Lbw, Lg, Rbw, Rg
         klist,                                                                  // int x N
         vb1c, vb2c,                                                             // int x N
         vb1s, vb2s,                                                             // u64 x N
@@ -230,15 +233,18 @@ Layout layout(int W, int H, size_t stride)
     L.N = (size_t)W * H;
     size_t o = 0;
     auto put = [&](int k, size_t bytes) { L.off[k] = o; o += (bytes + 255) / 256 * 256; };
-    for (int k = Layout::Lbw; k <= Layout::nrm; k++) put(k, L.N * 16);
+    for (int k = Layout::Lbw; k <= Layout::mR1; k++) put(k, L.N * 16);
+    auto share = [&](int k, int with) { L.off[k] = L.off[with]; };
+    share(Layout::chk, Layout::tmp);
+    share(Layout::nrm, Layout::mL1);
+    share(Layout::pself, Layout::Lbw);
+    share(Layout::pnb, Layout::Lg);
+    share(Layout::pselfR, Layout::Rbw);
+    share(Layout::pnbR, Layout::Rg);
     put(Layout::vb1c, L.N * 4);
     put(Layout::vb2c, L.N * 4);
     put(Layout::vb1s, L.N * 8);
     put(Layout::vb2s, L.N * 8);
-    put(Layout::pself, L.N * 16);
-    put(Layout::pnb, L.N * 16);
-    put(Layout::pselfR, L.N * 16);
-    put(Layout::pnbR, L.N * 16);
     put(Layout::klist, L.N * 4);
     put(Layout::texL, tex_bytes(W, H));
     put(Layout::texR, tex_bytes(W, H));

@@ -164,3 +164,28 @@ def test_branch_counts_and_autotuner_keep_results(torch_cuda, native):
         pm.set_batch_branches(99)
     with pytest.raises(_lib.StereoError):
         pm.set_batch_schedule("lockstep", 0, 0, 24)
+
+
+def test_workspace_per_pixel(torch_cuda):
+    """A single call, a depth_map call and a batch take at most 608 bytes a pixel of device memory for their
+    workspaces: what fits a device stays a matter of that figure.  (Inputs and kernels are loaded before;
+    64 MiB for outputs, graphs and allocation granularity.)"""
+    from cvt_b200 import PMHuberStereo
+
+    torch = torch_cuda
+    img = torch.zeros((1000, 1600, 4), dtype=torch.uint8, device="cuda")
+    calls = {"single": lambda pm, a, n: pm.disparity_map(a, a, 0, 4.0, 1),
+             "depth": lambda pm, a, n: pm.depth_map(a, a, 0, 4.0, 1),
+             "batch": lambda pm, a, n: pm.disparity_map_batch([a] * n, [a] * n, [0] * n, [4.0] * n, 1)}
+    for name, call in calls.items():
+        n = 2 if name == "batch" else 1
+        call(PMHuberStereo(), img[:200].contiguous(), n)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        pm = PMHuberStereo()
+        call(pm, img, n)
+        torch.cuda.synchronize()
+        used = free - torch.cuda.mem_get_info()[0]
+        assert used <= 608 * 1600 * 1000 * n + (64 << 20), (name, used / (1600 * 1000 * n))
+        del pm
