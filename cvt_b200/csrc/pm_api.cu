@@ -1753,12 +1753,14 @@ int pm_k_propagate(float* out, const float* old, const float* bw1, const float* 
     P.vout_src = (unsigned long long*)vout_src;
     P.counters = (unsigned long long*)counters;
     P.error = d_err;
+    const size_t N = (size_t)W * H;
     float4* tmp = nullptr;
-    PM_CUDA(nullptr, cudaMallocAsync((void**)&tmp, (size_t)W * H * 2 * sizeof(float4), S(stream)));
-    P.list = nullptr;
-    P.list_count = nullptr;
+    PM_CUDA(nullptr, cudaMallocAsync((void**)&tmp, N * (2 * sizeof(float4) + sizeof(int)) + sizeof(int), S(stream)));
     P.tmp_self = tmp;
-    P.tmp_nb = tmp + (size_t)W * H;
+    P.tmp_nb = tmp + N;
+    P.list = reinterpret_cast<int*>(tmp + 2 * N);
+    P.list_count = P.list + N;
+    cudaMemsetAsync(P.list_count, 0, sizeof(int), S(stream));   // an error shows below
     launch_propagate(P, fused, S(stream));
     PM_CUDA(nullptr, cudaFreeAsync(tmp, S(stream)));
     PM_CUDA(nullptr, cudaGetLastError());

@@ -35,13 +35,13 @@ struct PropParams {
     unsigned long long* counters;   // null: not counted
     int* error;                     // incremented if a view-buffer insert gave up
     // per-pixel state between the three propagate kernels: the plane after the candidates and its Gauss-Newton
-    // result; with `list` they are this view's own and still hold the previous iteration's
+    // result; if `known` they are this view's own and still hold the previous iteration's
     float4* tmp_self;
     float4* tmp_nb;
-    int* list;                      // may be null: pixels whose Gauss-Newton steps are to be run, and their
-    int* list_count;                // number (0 between passes)
+    int* list;                      // pixels whose Gauss-Newton steps are to be run (unused by the batched and the
+    int* list_count;                // counted kernels), and their number (0 between passes)
     int dual;                       // the window-loop kernels run as two variants (pm_window.cuh)
-    int known;                      // the costs in `old` are those of its planes (k_prop_chain)
+    int known;                      // a pass within a run: the costs in `old` are those of its planes (k_prop_chain)
     int owners;                     // pixels per warp row of the propagate kernels (set by the launchers)
 };
 

@@ -1,8 +1,8 @@
 // pmhstereo_propagate_view (cvt/cl/kernel/pmhstereo.cl:880-1071) on sm_100a, as three
 // kernels over the same pixels:
 //   k_prop_chain  the candidate chain up to the randomized refinement (:927-1028)
-//   k_prop_klt    the six Gauss-Newton steps (:1034-1038); k_prop_klt_list runs them for listed pixels,
-//                 k_prop_klt_warp with few pixels per warp
+//   k_prop_klt_list  the six Gauss-Newton steps (:1034-1038) of listed pixels; k_prop_klt_warp runs them with few
+//                 pixels per warp, k_prop_klt over the general loops
 //   k_prop_final  the evaluation of their result, the view scatter and the output (:1039-1070)
 // The state between them is `self` and the Gauss-Newton result (two float4 fields).
 //
@@ -190,12 +190,12 @@ __device__ __forceinline__ void chain_tile(const PropParams& P, WarpScratch<>* w
             sd_self = sd;
         }
     }
-    // Within a run the Gauss-Newton steps of a plane that the pixel already had after the previous iteration's
-    // candidates would give the result that still lies in tmp_nb.  The others are listed, a warp's pixels
-    // together (launch_pass; the list's order changes nothing, each pixel is on its own).
+    // Within a run (P.known) the Gauss-Newton steps of a plane that the pixel already had after the previous
+    // iteration's candidates would give the result that still lies in tmp_nb.  The others are listed, a warp's
+    // pixels together (launch_pass; the list's order changes nothing, each pixel is on its own).
     if (!GEN && P.list) {
         bool todo = own;
-        if (own && P.iter > 0) {
+        if (own && P.known && P.iter > 0) {
             const float4 was = P.tmp_self[idx];
             todo = __float_as_uint(was.x) != __float_as_uint(self.x) || __float_as_uint(was.y) != __float_as_uint(self.y) ||
                    __float_as_uint(was.z) != __float_as_uint(self.z);
@@ -234,16 +234,16 @@ __device__ __forceinline__ void klt_tile(const PropParams& P, int bx, int by, Co
     }
 }
 
-template <bool F, bool COUNT, bool GEN>
+template <bool F, bool COUNT>
 __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt(PropParams P)
 {
-    if (variant_skips<GEN>(P.V, P.dual)) return;
+    if (variant_skips<true>(P.V, P.dual)) return;
     Counters cnt = {0, 0, 0, 0};
-    klt_tile<F, COUNT, GEN>(P, blockIdx.x, blockIdx.y, cnt);
+    klt_tile<F, COUNT, true>(P, blockIdx.x, blockIdx.y, cnt);
     flush_counters<COUNT>(cnt, P.counters);
 }
 
-// the same for the pixels of P.list
+// the same over the pair-plane loops, for the pixels of P.list
 template <bool F>
 __global__ void __launch_bounds__(PROP_THREADS, PM_KLT_BLOCKS) k_prop_klt_list(PropParams P)
 {
@@ -499,9 +499,8 @@ void launch_pass(const PropParams& Q, cudaStream_t st)
     k_prop_chain<F, false, false><<<g, b, 0, st>>>(Q);
     k_prop_chain<F, false, true><<<gg, b, 0, st>>>(G);
     if (Q.owners <= WARP_KLT) k_prop_klt_warp<F><<<g, b, 0, st>>>(Q);
-    else if (Q.list) k_prop_klt_list<F><<<(Q.V.W * Q.V.H + PROP_THREADS - 1) / PROP_THREADS, PROP_THREADS, 0, st>>>(Q);
-    else k_prop_klt<F, false, false><<<gg, b, 0, st>>>(G);
-    k_prop_klt<F, false, true><<<gg, b, 0, st>>>(G);
+    else k_prop_klt_list<F><<<(Q.V.W * Q.V.H + PROP_THREADS - 1) / PROP_THREADS, PROP_THREADS, 0, st>>>(Q);
+    k_prop_klt<F, false><<<gg, b, 0, st>>>(G);
     k_prop_final<F, false, false><<<g, b, 0, st>>>(Q);
     k_prop_final<F, false, true><<<gg, b, 0, st>>>(G);
 }
@@ -513,7 +512,7 @@ void launch_pass_counted(const PropParams& Q, cudaStream_t st)
     const dim3 b(PROP_BX, PROP_BY);
     const dim3 g = grid2d(Q.V.W, Q.V.H, b);
     k_prop_chain<F, true, true><<<g, b, 0, st>>>(Q);
-    k_prop_klt<F, true, true><<<g, b, 0, st>>>(Q);
+    k_prop_klt<F, true><<<g, b, 0, st>>>(Q);
     k_prop_final<F, true, true><<<g, b, 0, st>>>(Q);
 }
 

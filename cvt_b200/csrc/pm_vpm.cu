@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(PT, 5) k_cand(float4* __restrict__ cur_out, co
     }
     if (list) {
         bool todo = P.own;
-        if (P.own && iter > 0) {
+        if (P.own && known && iter > 0) {
             const float4 was = prev[P.i];
             todo = __float_as_uint(was.x) != __float_as_uint(cur.x) || __float_as_uint(was.y) != __float_as_uint(cur.y) ||
                    __float_as_uint(was.z) != __float_as_uint(cur.z);
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(PT, 5) k_steps_list(float4* __restrict__ out, 
     out[idx] = s;
 }
 
-// the evaluation of their result (:350-358), as k_settle
+// the evaluation of their result (:350-358); out holds the candidates' state
 __global__ void __launch_bounds__(PT, 5) k_settle_list(float4* __restrict__ out, const float4* __restrict__ steps, Views V,
                                                     const int* __restrict__ list)
 {
@@ -406,28 +406,20 @@ __global__ void __launch_bounds__(PT, 5) k_settle_list(float4* __restrict__ out,
     if (own && s.w < cur.w) out[idx] = s;
 }
 
-// three Gauss-Newton steps (:347-349), a thread per pixel or, on small images, a few pixels per warp
-template <bool SHARED>
+// the steps with a few pixels per warp (owners <= WARP_KLT), every pixel
 __global__ void __launch_bounds__(PT, 5) k_steps(float4* __restrict__ out, const float4* __restrict__ cur, Views V,
                                               int owners)
 {
     if (variant_skips<false>(V, 1)) return;
-    __shared__ WarpScratch<VPM> ws[SHARED ? PT / 32 : 1];
+    __shared__ WarpScratch<VPM> ws[PT / 32];
     const VPixel P(V, owners);
-    if (SHARED) {
-        if (P.y >= V.H) return;   // a whole warp
-        float4 s = P.own ? __ldg(cur + P.i) : f4(0.0f, 0.0f, 0.0f, 0.0f);
-        s = klt2_steps_warp<false, VPM>(V, ws[threadIdx.y], P.lane, owners, 3, P.own, P.x, P.y, s);
-        if (P.own) out[P.i] = s;
-    } else if (P.own) {
-        float4 s = __ldg(cur + P.i);
-#pragma unroll 1
-        for (int k = 0; k < 3; k++) s = klt2_pair<false, VPM>(V, P.x, P.y, s);
-        out[P.i] = s;
-    }
+    if (P.y >= V.H) return;   // a whole warp
+    float4 s = P.own ? __ldg(cur + P.i) : f4(0.0f, 0.0f, 0.0f, 0.0f);
+    s = klt2_steps_warp<false, VPM>(V, ws[threadIdx.y], P.lane, owners, 3, P.own, P.x, P.y, s);
+    if (P.own) out[P.i] = s;
 }
 
-// the evaluation of their result (:350-358); out holds the candidates' state
+// and the evaluation of their result
 __global__ void __launch_bounds__(PT, 5) k_settle(float4* __restrict__ out, const float4* __restrict__ steps, Views V,
                                                int owners)
 {
@@ -473,8 +465,8 @@ void launch_init(float4* out, const Views& V, float dmax, const float* initdisp,
     k_init<<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, V, dmax, initdisp);
 }
 
-// one pass from `in` to `out`; steps: a W*H field.  known: a run, every state's cost is its plane's; prev
-// and list (W*H planes, W*H + 1 ints) then hold what k_cand keeps from one iteration to the next
+// one pass from `in` to `out`; steps: a W*H field; prev and list (W*H planes, W*H + 1 ints): what k_cand keeps.
+// known: an iteration of a run, every state's cost is its plane's and prev holds the previous iteration's
 void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, float dmax, int iter, int known,
                  float4* prev, int* list, unsigned long long* counts, cudaStream_t st)
 {
@@ -484,7 +476,7 @@ void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, f
     }
     const int owners = prop_owners(V.W, V.H);
     const dim3 b(32, PT / 32), g((V.W + owners - 1) / owners, (V.H + PT / 32 - 1) / (PT / 32));
-    if (known && owners > WARP_KLT) {
+    if (owners > WARP_KLT) {
         const int blocks = (int)(((size_t)V.W * V.H + PT - 1) / PT);
         cudaMemsetAsync(list, 0, sizeof(int), st);
         k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known, prev, list);
@@ -492,8 +484,7 @@ void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, f
         k_settle_list<<<blocks, PT, 0, st>>>(out, steps, V, list);
     } else {
         k_cand<<<g, b, 0, st>>>(out, in, V, dmax, iter, owners, known, nullptr, nullptr);
-        if (owners <= WARP_KLT) k_steps<true><<<g, b, 0, st>>>(steps, out, V, owners);
-        else k_steps<false><<<g, b, 0, st>>>(steps, out, V, owners);
+        k_steps<<<g, b, 0, st>>>(steps, out, V, owners);
         k_settle<<<g, b, 0, st>>>(out, steps, V, owners);
     }
     k_iter<false><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, nullptr);
@@ -630,10 +621,11 @@ int run_simple(pm_vpm* h, const uint8_t* img0, const uint8_t* img1, int W, int H
 }
 
 // the texel planes from the reference kernels' inputs (RGBA8 colour images and float4 gradient
-// images), in stream-ordered scratch, with a W*H field for the Gauss-Newton results
+// images), in stream-ordered scratch, with a pass's fields (launch_iter)
 struct VpmScratch {
     float4* p = nullptr;
-    float4* steps = nullptr;
+    float4 *steps = nullptr, *prev = nullptr;
+    int* list = nullptr;
     cudaStream_t st = nullptr;
     ~VpmScratch()
     {
@@ -644,9 +636,11 @@ struct VpmScratch {
     {
         st = s;
         const size_t N = (size_t)W * H, T = tex_bytes(W, H) / sizeof(float4);
-        VPM_CUDA(nullptr, cudaMallocAsync((void**)&p, (2 * T + 2 * N) * sizeof(float4), s));
+        VPM_CUDA(nullptr, cudaMallocAsync((void**)&p, (2 * T + 2 * N) * sizeof(float4) + (N + 1) * sizeof(int), s));
         steps = p + 2 * T;
-        launch_views(p, p + T, steps, steps + N, c1, c2, reinterpret_cast<const float4*>(g1),
+        prev = steps + N;
+        list = reinterpret_cast<int*>(prev + N);
+        launch_views(p, p + T, steps, prev, c1, c2, reinterpret_cast<const float4*>(g1),
                      reinterpret_cast<const float4*>(g2), W, H, stride, r, s);
         *V = make_view(p, p + T, W, H, r);
         return PM_OK;
@@ -800,8 +794,8 @@ int pm_k_vpm_iter(float* out, const float* in, const uint8_t* c1, const float* g
     Views V;
     rc = sc.make(c1, g1, c2, g2, W, H, stride, r, S(stream), &V);
     if (rc) return rc;
-    launch_iter(reinterpret_cast<float4*>(out), reinterpret_cast<const float4*>(in), sc.steps, V, dmax, iter, 0, nullptr,
-                nullptr, nullptr, S(stream));
+    launch_iter(reinterpret_cast<float4*>(out), reinterpret_cast<const float4*>(in), sc.steps, V, dmax, iter, 0, sc.prev,
+                sc.list, nullptr, S(stream));
     VPM_CUDA(nullptr, cudaGetLastError());
     return PM_OK;
 }

@@ -12,8 +12,9 @@ from oracle.pyoracle import bits_equal
 
 pytestmark = pytest.mark.gpu
 
-# (width, height, patch half-width, disparity range, planes)
-PAIRS = [(72, 40, 3, 16.0, 5), (40, 56, 2, 12.0, 4), (96, 33, 4, 24.0, 6), (33, 17, 1, 8.0, 3)]
+# (width, height, patch half-width, disparity range, planes); the last is above the 11,840 pixels from which single
+# pairs run the Gauss-Newton steps over a list of changed planes
+PAIRS = [(72, 40, 3, 16.0, 5), (40, 56, 2, 12.0, 4), (96, 33, 4, 24.0, 6), (33, 17, 1, 8.0, 3), (151, 101, 3, 20.0, 6)]
 
 
 @pytest.fixture(scope="module")

@@ -396,6 +396,31 @@ def test_pipeline_fused_matches_oracle(native, torch_cuda, orc, W, H, r, dmax, i
     assert pm.counters() == [int(v) for v in ctr], "window-sample counts equal the oracle's"
 
 
+@pytest.mark.parametrize("entry,fused,views,pp", [("disparity", 0, 2, 1), ("disparity", 1, 2, 2), ("disparity", 0, 1, 0),
+                                                  ("depth", 0, 2, 1), ("depth", 1, 2, 2), ("depth", 1, 1, 0),
+                                                  ("pyramid", 0, 2, 1), ("pyramid", 1, 2, 1)])
+def test_runs_over_changed_planes_match_oracle(native, torch_cuda, orc, entry, fused, views, pp):
+    """Whole runs above the size where the Gauss-Newton steps go over the list of changed planes (11,840 pixels;
+    the finer of the pyramid's two levels), with enough iterations for planes to settle:
+    disparity map, depth map and pyramid, each view's own stored results."""
+    from cvt_b200 import PMHuberStereo, scene
+
+    W, H, r, dmax, iters = 151, 101, 4, 24.0, 5
+    L, R = scene.generate(31 + views, W, H, 8, 2.0, dmax - 2.0)
+    kw, levels = dict(pp=pp, views=views, fused=fused), 2 if entry == "pyramid" else 1
+    pm = PMHuberStereo(fused=bool(fused), views=views, levels=levels)
+    if entry == "depth":
+        o, run = orc.depth_map(L, R, r, dmax, iters, **kw), pm.depth_map
+    else:
+        o, run = orc.disparity_map(L, R, r, dmax, iters, levels=levels, **kw), pm.disparity_map
+    res = run(L, R, r, dmax, iters, pp=pp, normalmap=True, planes=True)
+    assert bits_equal(res["planes_left"], o["planesL"]).all()
+    if views == 2:
+        assert bits_equal(res["planes_right"], o["planesR"]).all()
+    assert bits_equal(res["dmap"], o["dmap"]).all()
+    assert bits_equal(res["normal"], o["normal"]).all()
+
+
 @pytest.mark.parametrize("W,H,r,dmax,iters,seed", [(4096, 6, 10, 64.0, 2, 3), (72, 40, 32, 24.0, 2, 4),
                                                     (5, 4096, 3, 4.0, 1, 5)])
 def test_maximum_width_height_and_radius_match_oracle(native, torch_cuda, orc, W, H, r, dmax, iters, seed):
