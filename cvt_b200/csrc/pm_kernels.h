@@ -157,7 +157,7 @@ inline ViewData make_view(const float4* t1, const float4* t2, int W, int H, int 
 {
     const int plane = tex_pitch(W) * H;
     return ViewData{t1, t2, W, H, r, tex_pitch(W), plane, reinterpret_cast<const int*>(t1 + (size_t)TEX_PLANES * plane),
-                    reinterpret_cast<const int*>(t2 + (size_t)TEX_PLANES * plane)};
+                    reinterpret_cast<const int*>(t2 + (size_t)TEX_PLANES * plane), WindowSpan(W, H, r, W, H)};
 }
 void launch_pack_tex(float4* tex, const float4* bw, const float4* grad, int W, int H, int fused, cudaStream_t st);
 // FP32 peak probe: `iters` rounds of independent fma chains per thread

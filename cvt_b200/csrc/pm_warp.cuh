@@ -41,22 +41,19 @@ struct WarpItem {
     }
 };
 
-// sample e of a window of L columns: row (e recip) >> 20 with recip = ceil(2^20 / L), exact for e < L^2, L <= 65
-__device__ __forceinline__ int window_row(int e, unsigned recip) { return (int)(((unsigned)e * recip) >> 20); }
-
 // Samples e0 .. e0 + len - 1 of the windows of patch_eval_census of the n pixels whose parameters are in S.par,
 // spread over the warp; their terms go to S.term[task * len + sample - e0].  ROW: all windows
 // have the top row `top` (a warp along an image row).
 template <bool F, bool ROW, Model M>
 __device__ __forceinline__ void eval_terms_shared(const ViewData& V, WarpScratch<M>& S, int lane, int n, int e0, int len,
-                                                  unsigned recip, int top)
+                                                  const WindowSpan& span, int top)
 {
-    const int W = V.W, L = 2 * V.r + 1;
+    const int W = V.W;
     const float fW = (float)W;
     for (WarpItem it(lane, e0, len); it.i < n * len; it.next()) {
         const float4 A = S.par[it.task][0], B = S.par[it.task][1];   // (s.x, s.y, s.z, left column), (colour, top row)
-        const int e = it.e0 + it.e, j = window_row(e, recip);
-        const int y = (ROW ? top : __float_as_int(B.w)) + j, x = __float_as_int(A.w) + e - j * L;
+        const int e = it.e0 + it.e, j = span.row(e);
+        const int y = (ROW ? top : __float_as_int(B.w)) + j, x = __float_as_int(A.w) + e - j * span.cols;
         const bool in1 = (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)V.H;
         const int yc = min(max(y, 0), V.H - 1);
         const float qx = (float)x;
@@ -109,26 +106,29 @@ __device__ __forceinline__ float patch_eval_warp(const ViewData& V, WarpScratch<
         in = __ldg(V.row1(py) + px);
         thr = exit_threshold(mincost, in.w);
     }
-    const int r = V.r, L = 2 * r + 1, top = py - r;
+    const int r = V.r;
     const float qx0 = (float)max(px - r, 0), qx1 = (float)min(px + r, V.W - 1);
-    const unsigned recip = ((1u << 20) + L - 1) / L;
-    for (int e0 = 0; e0 < L * L;) {
+    // constant operands (V.span) are 0.7% faster in the main path's candidate kernel (320x240, r = 7) and up to
+    // 6% slower in VPM's (107x110, r = 10)
+    const WindowSpan span = M == PMH ? V.span : WindowSpan(V.W, V.H, r, V.W, V.H);
+    const int top = span.top(py, r), left = span.left(px, r), samples = span.cols * span.rows;
+    for (int e0 = 0; e0 < samples;) {
         const unsigned m = __ballot_sync(0xffffffffu, act);
         const int n = __popc(m);
         if (n == 0) break;
         if (n > WARP_TASKS) {   // every lane its own row
-            const int iy = top + window_row(e0, recip);
+            const int iy = top + span.row(e0);
             if (act && iy >= 0 && iy < V.H) eval_row_pixel<F, M>(V, iy, s, s.y * (float)iy, in, qx0, qx1, census, wsum);
-            e0 += L;
+            e0 += span.cols;
         } else {
             const int rank = __popc(m & ((1u << lane) - 1u));
-            const int len = min((WARP_TERMS / n - 1) | 1, L * L - e0);   // odd: the ordered sums read with this stride
+            const int len = min((WARP_TERMS / n - 1) | 1, samples - e0);   // odd: the ordered sums read with this stride
             if (act) {
-                S.par[rank][0] = f4(s.x, s.y, s.z, __int_as_float(px - r));
+                S.par[rank][0] = f4(s.x, s.y, s.z, __int_as_float(left));
                 S.par[rank][1] = f4(in.x, in.y, in.z, __int_as_float(top));
             }
             __syncwarp();
-            eval_terms_shared<F, ROW, M>(V, S, lane, n, e0, len, recip, top);
+            eval_terms_shared<F, ROW, M>(V, S, lane, n, e0, len, span, top);
             __syncwarp();
             if (act) {
                 const float2* v = S.term + rank * len;
@@ -161,11 +161,12 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
                                                   bool need, int px, int py, float4 s)
 {
     constexpr int NU = (9 * WARP_KLT + 31) / 32;   // sums per lane, at most
-    const int W = V.W, r = V.r, L = 2 * r + 1, top = py - r;
+    const int W = V.W, r = V.r;
     const int units = 9 * owners;
-    const unsigned recip = ((1u << 20) + L - 1) / L;
+    const WindowSpan span(W, V.H, r, W, V.H);   // V.span's constant operands: 1-3% slower (64x48, r = 32)
+    const int cols = span.cols, top = span.top(py, r);
     // rows inside the image: samples first .. end - 1
-    const int first = max(-top, 0) * L, end = min(L, V.H - top) * L;
+    const int first = max(-top, 0) * cols, end = min(span.rows, V.H - top) * cols;
     float* const sums = reinterpret_cast<float*>(S.term);
     const float4 c1 = need ? __ldg(V.row1(py) + px) : f4(0.0f, 0.0f, 0.0f, 0.0f);
     const int chunk = WARP_TERMS / owners;
@@ -174,7 +175,7 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
         const bool nan = s.x != s.x || s.y != s.y || s.z != s.z;
         const unsigned m = __ballot_sync(0xffffffffu, need && !nan);
         if (lane < owners) {
-            S.par[lane][0] = f4(s.x, s.y, s.z, (float)(px - r));
+            S.par[lane][0] = f4(s.x, s.y, s.z, (float)span.left(px, r));
             S.par[lane][1] = f4(c1.x, c1.y, c1.z, 0.0f);
         }
         float acc[NU];
@@ -186,8 +187,8 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
             for (WarpItem it(lane, e0, len); it.i < owners * len; it.next()) {
                 float2 v = f2(0.0f, 0.0f);
                 const float4 A = S.par[it.task][0];
-                const int e = it.e0 + it.e, j = window_row(e, recip), y = top + j;
-                const float qx = A.w + (float)(e - j * L);
+                const int e = it.e0 + it.e, j = span.row(e), y = top + j;
+                const float qx = A.w + (float)(e - j * cols);
                 // the 3-point cost needs 1 <= qx < W - 1
                 if (((m >> it.task) & 1u) && qx >= 1.0f && qx < (float)(W - 1)) {
                     const float4 c = S.par[it.task][1];
@@ -208,12 +209,12 @@ __device__ __forceinline__ float4 klt2_steps_warp(const ViewData& V, WarpScratch
                     const float* v = reinterpret_cast<const float*>(S.term + task * len) + (j >= 3);
                     const float left = S.par[task][0].w;
                     float sum = acc[k];
-                    int row = window_row(e0, recip), dx = e0 - row * L;
+                    int row = span.row(e0), dx = e0 - row * cols;
                     for (int d = 0; d < len;) {
                         const float qy = (float)(top + row);
                         const float f1 = fx ? 1.0f : 0.0f, f0 = fx ? 0.0f : fy ? qy : 1.0f;
                         const float g1 = gx ? 1.0f : 0.0f, g0 = gx ? 0.0f : gy ? qy : 1.0f;
-                        const int stop = min(len, d + L - dx);
+                        const int stop = min(len, d + cols - dx);
                         float qx = left + (float)dx;
 #pragma unroll 4
                         for (; d < stop; d++, qx += 1.0f) {

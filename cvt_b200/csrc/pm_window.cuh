@@ -35,6 +35,26 @@ namespace pm {
 constexpr int TEX_PAD = 4;     // replicated columns on each side of a texel row
 constexpr int TEX_PLANES = 4;  // colour, gradient, compact, pair
 
+// The samples over which a warp walks the windows it shares (pm_warp.cuh), row by row: the 2 r + 1 columns and rows
+// from (px - r, py - r), those outside the image with weight 0; or, where the window of every pixel of the
+// PW x PH that have one spans the image (at most r + 1 columns or rows), the image's (17x9, r = 32: 153
+// samples a window, not 4225).
+struct WindowSpan {
+    int cols, rows;
+    unsigned recip;       // ceil(2^20 / cols): row(e) is exact for e < cols rows, both <= 65
+    int xmask, ymask;     // 0: all windows start at column (row) 0, else -1
+    __host__ __device__ WindowSpan(int W, int H, int r, int PW, int PH)
+        : cols(PW <= r + 1 ? W : 2 * r + 1), rows(PH <= r + 1 ? H : 2 * r + 1), recip(((1u << 20) + cols - 1) / cols),
+          xmask(PW <= r + 1 ? 0 : -1), ymask(PH <= r + 1 ? 0 : -1)
+    {
+    }
+    WindowSpan() = default;
+    __device__ __forceinline__ int row(int e) const { return (int)(((unsigned)e * recip) >> 20); }
+    // first column and row of a pixel's window
+    __device__ __forceinline__ int left(int px, int r) const { return (px - r) & xmask; }
+    __device__ __forceinline__ int top(int py, int r) const { return (py - r) & ymask; }
+};
+
 struct ViewData {
     const float4* __restrict__ t1;   // first view: colour plane, gradient at + plane, compact at + 2 plane, pair at + 3 plane
     const float4* __restrict__ t2;   // second view
@@ -42,6 +62,7 @@ struct ViewData {
     int plane;                       // H * P
     const int* gen1;                 // the views' flags: read by the general loops (after the planes)
     const int* gen2;
+    WindowSpan span;
     // colour texel (compact texel) of column 0 of row y
     __device__ __forceinline__ const float4* row1(int y) const { return t1 + (size_t)y * P + TEX_PAD; }
     __device__ __forceinline__ const float4* row1c(int y) const { return t1 + 2 * (size_t)plane + (size_t)y * P + TEX_PAD; }

@@ -291,7 +291,8 @@ def test_pair_plane_loops_match_oracle(D, orc, W, H, r, fused):
 
 
 @pytest.mark.parametrize("fused", [0, 1])
-@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 5), (148, 80, 3), (149, 80, 4), (33, 400, 1)])
+@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 5), (148, 80, 3), (149, 80, 4), (33, 400, 1),
+                                   (5, 9, 4), (6, 5, 4)])
 def test_propagate_over_pair_planes_matches_oracle(D, orc, W, H, r, fused):
     """One propagate pass from the planes of pair_planes: two, four and 32 pixels per warp (the bounds of
     prop_owners among the sizes), windows of several passes over the shared memory, shared and single rows
@@ -756,3 +757,40 @@ def test_small_config_strict_exact_fused_within_tolerance(native, torch_cuda, or
     within = same | ((dd <= 1e-3) & (rc <= 1e-4))
     print("fused vs reference, 320x240: planes equal %.4f, within tolerance %.4f" % (same.mean(), within.mean()))
     assert within.mean() > 0.8 and (dd < 1.0).mean() > 0.97
+
+
+def test_windows_larger_than_the_image(native, torch_cuda):
+    """Where every window spans the image, a larger window is the same call: the same results, and not the time of
+    the samples outside the image (3 times allowed; all of them would be 10 times and more)."""
+    import statistics
+
+    from cvt_b200 import PMHuberStereo, scene
+    from cvt_b200.svpm import SVPMFlowCL
+    from cvt_b200.vpm import VPMStereoCL
+
+    torch = torch_cuda
+
+    def timed(call):
+        out = call()
+        ms = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            out = call()
+            b.record()
+            torch.cuda.synchronize()
+            ms.append(a.elapsed_time(b))
+        return host(out), statistics.median(ms)
+
+    for size, small in ((9, 8), (16, 15)):
+        a, b = (dev(torch, i) for i in scene.generate(5, size, size, 3, 0.5, 3.0))
+        stereo, flow = PMHuberStereo(), SVPMFlowCL()
+        calls = {"disparity": lambda r: stereo.disparity_map(a, b, r, 8.0, 3),
+                 "depth": lambda r: stereo.depth_map(a, b, r, 8.0, 3),
+                 "vpm": lambda r, h={r: VPMStereoCL(r, 8, 8.0) for r in (small, 32)}: h[r].disparity_simple(a, b)}
+        if size == 16:   # the flow's pixels are those of 16x16 groups
+            calls["flow"] = lambda r: flow.flow(a, b, r, 4.0, 12)
+        for name, call in calls.items():
+            (few, t0), (all32, t1) = timed(lambda: call(small)), timed(lambda: call(32))
+            assert bits_equal(few, all32).all(), (size, name)
+            assert t1 < 3.0 * t0, (size, name, t0, t1)

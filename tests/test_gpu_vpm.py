@@ -95,7 +95,8 @@ def test_vpm_kernels_match_reference_golden(torch_cuda, native, case):
 
 
 @pytest.mark.parametrize("finite", [True, False])
-@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 3), (149, 80, 4)])
+@pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 3), (149, 80, 4), (5, 9, 4),
+                                   (6, 5, 4)])
 def test_vpm_iteration_over_pair_planes_matches_oracle(torch_cuda, native, orc, W, H, r, finite):
     """One pass from the planes of pair_planes with costs that are not the planes': two, four and 32 pixels per
     warp; with first-image gradients that are not finite, the general loops.  (Infinite second-image gradients
