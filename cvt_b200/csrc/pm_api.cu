@@ -53,6 +53,8 @@ struct pm_handle {
     const float* init_normal_right = nullptr;   // with init_right: the right view's initial normals
     // concurrent branches of batched calls (pm_set_batch_branches; 0: PM_BATCH_BRANCHES)
     int batch_branches = 0;
+    // pixels that a branched batch in progress runs at a time, 0 otherwise (PropParams::load)
+    int batch_load = 0;
     // schedule of batched calls (pm_set_batch_schedule)
     int batch_schedule = PM_BATCH_BRANCHED, batch_ctas = 0, batch_order = 0, batch_tile_w = 32;
     // lockstep batched calls: per-pair argument tables, job lists and work counters in one
@@ -381,6 +383,7 @@ PropParams prop_params(const pm_handle* h, const LevelBufs& B, int view, int ite
     P.list_count = B.kcount;
     P.dual = 0;
     P.known = 1;
+    P.load = h->batch_load;
     return P;
 }
 
@@ -582,6 +585,7 @@ int run_depth(pm_handle* h, void* ws, const uint8_t* left, const uint8_t* right,
         P.list_count = at<int>(ws, L, Layout::kcount);
         P.dual = 0;
         P.known = 1;
+        P.load = 0;
         launch_propagate(P, F, st);   // :263-264
         if (views == 2) {
             P.tmp_self = at<float4>(ws, L, Layout::pselfR);
@@ -1621,6 +1625,14 @@ int pm_disparity_map_batch_device(pm_handle* h, int n, const uint8_t* const* lef
             return rc;
         }
     }
+    // one pair's pixels on each branch, the other branches' for nine tenths: pairs also wait between their passes
+    double px = 0.0;
+    for (int i = 0; i < n; i++) px += (double)width[i] * height[i];
+    struct Load {
+        pm_handle* h;
+        ~Load() { h->batch_load = 0; }
+    } load{h};
+    h->batch_load = (int)(px / n * (1.0 + 0.9 * (nb - 1)));
     auto body = [&](cudaStream_t cs) -> int {
         PM_CUDA(h, cudaEventRecord(h->bev[nb], cs));
         for (int b = 0; b < nb; b++) PM_CUDA(h, cudaStreamWaitEvent(h->branch[b], h->bev[nb], 0));
@@ -1744,6 +1756,7 @@ int pm_k_propagate(float* out, const float* old, const float* bw1, const float* 
     P.theta = theta;
     P.dmax = dmax;
     P.known = 0;
+    P.load = 0;
     P.lr = lr;
     P.iter = iter;
     P.vin_count = vin_count;

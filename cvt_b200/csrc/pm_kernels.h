@@ -43,6 +43,7 @@ struct PropParams {
     int dual;                       // the window-loop kernels run as two variants (pm_window.cuh)
     int known;                      // a pass within a run: the costs in `old` are those of its planes (k_prop_chain)
     int owners;                     // pixels per warp row of the propagate kernels (set by the launchers)
+    int load;                       // pixels of this and the passes that run beside it, if more than its own (prop_owners)
 };
 
 // Batched launches over many pairs (pm_disparity_map_batch_device run in lockstep): a job is
@@ -114,8 +115,8 @@ void launch_init(float4* out, const ViewData& V, float dmax, int lr, const float
 void launch_cost(float* cost, const float4* planes, const ViewData& V, float mincost, int fused, cudaStream_t st);
 void launch_klt(float4* out, const float4* planes, const ViewData& V, int fused, cudaStream_t st);
 void launch_propagate(const PropParams& P, int fused, cudaStream_t st);
-// pixels per warp of a window pass over one W x H image (pm_propagate.cu)
-int prop_owners(int W, int H);
+// pixels per warp of a window pass when `pixels` pixels run at a time, other pairs' beside it (pm_propagate.cu)
+int prop_owners(long long pixels, int r, Model m, bool beside);
 // launches per window-loop kernel (init, cost, klt, each of the three propagate kernels):
 // uncounted runs launch both variants (pm_window.cuh)
 inline int window_kernel_launches(int fused, bool counting)

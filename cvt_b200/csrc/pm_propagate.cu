@@ -471,18 +471,31 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
     }
 }
 
-// Pixels per warp of a single-pair pass over W x H pixels: a thread per pixel (32) unless the image is so
-// small that its warps, one thread's serial windows each, leave the chip idle.  Measured, ms a
-// call (two views, 5 iterations) with 32 / 16 / 8 / 4 / 2 / 1 pixels: 64x48, r = 5: - / - / 4.10 / 3.42 /
-// 3.00 / 3.44; 80x60, r = 7: - / 9.17 / 5.81 / 4.80 / 4.41 / 5.20; 120x90, r = 10: 13.8 / 18.1 / 12.1 / 10.2 /
-// 10.5 / -; 120x90, r = 3: 3.60 / 4.18 / 3.48 / 3.37 / 3.86 / -; 160x120, r = 7: 8.2 / 11.7 / 9.7 / 9.5;
-// 220x160, r = 5: 6.7 / 9.2 / 9.7.  Shared windows take 1.6 times the instructions, so they win only while
-// about 3000 warps (20 per SM) hold the image with at most 4 pixels each.
-int prop_owners(int W, int H)
+// Pixels per warp of a pass when `pixels` pixels run at a time, windows of half-width r: a thread per pixel (32)
+// unless the pixels are so few that their warps, one thread's serial windows each, leave the chip idle.
+// Shared windows take 1.6 times the instructions, and small ones do not fill a warp's rows, so they win only while
+// about 20 warps per SM (WARPS) hold the pixels with 2 or 4 each.
+// Measured, ms a call with 2 / 4 / 32 pixels, disparity maps of 5 iterations (two views) and VPM of 4:
+//            64x48               90x68               107x110             160x120             181x130
+//   r = 1    1.40 / 1.42 / 1.58  1.79 / 1.49 / 1.60  2.38 / 2.00 / 1.65  3.13 / 2.39 / 1.73  3.60 / 2.76 / 1.77
+//   r = 3    1.69 / 1.81 / 2.60  2.30 / 1.97 / 2.64  3.19 / 2.79 / 2.75  4.42 / 3.58 / 2.85  5.14 / 4.16 / 3.00
+//   r = 5    2.12 / 2.49 / 4.36  3.00 / 2.81 / 4.45  4.37 / 4.00 / 4.57  6.22 / 5.45 / 4.81  7.35 / 6.48 / 5.26
+//   r = 10   4.12 / 5.36 / 12.2  6.19 / 6.50 / 12.4  9.93 / 9.47 / 13.3  14.8 / 14.0 / 14.0  17.6 / 16.7 / 16.0
+//   VPM 1    0.20 / 0.22 / 0.31  0.27 / 0.23 / 0.30  0.38 / 0.32 / 0.31  0.50 / 0.39 / 0.32  0.59 / 0.46 / 0.33
+//   VPM 5    0.48 / 0.60 / 1.49  0.72 / 0.67 / 1.47  1.09 / 0.99 / 1.55  1.59 / 1.40 / 1.65  1.89 / 1.63 / 1.74
+//   VPM 10   1.26 / 1.66 / 4.67  1.91 / 1.95 / 4.61  3.03 / 2.87 / 4.77  4.53 / 4.24 / 5.36  5.35 / 4.90 / 5.51
+// Single runs stop at 4 WARPS, where the windows are large enough: the planes of a depth map settle, and the list
+// of changed ones is then worth more than sharing (115x115, 9 iterations, 4 / 32 pixels: r = 5 8.9 / 6.9 ms, r = 10
+// 16.7 / 16.2; a disparity map 8.2 / 8.4, 19.5 / 24.4).  Pairs of a batch run side by side (`beside`; pm_api.cu,
+// batch_load): 32 pairs of 120x90, r = 7: 139 / 119 / 56.6; 16 of 64x48, r = 5: 13.9 / 12.2 / 7.3; 4: 4.2 / 3.8 / 4.8;
+// 2: 2.7 / 2.9 / 4.6; 100x80, r = 10, 4 pairs: 21.8 / 19.6 / 18.1, 2: 11.6 / 11.0 / 13.5.
+int prop_owners(long long pixels, int r, Model m, bool beside)
 {
-    constexpr long long WARPS = 2960;
-    const long long n = (long long)W * H;
-    return n <= 2 * WARPS ? 2 : n <= 4 * WARPS ? 4 : 32;
+    constexpr float WARPS = 2960.0f;
+    const float n = (float)pixels / WARPS;
+    float four = beside ? fminf(fmaxf(2.2f + 0.48f * r, 4.0f), 10.0f) : 4.0f;
+    if (m == PMH) four = fminf(four, 2.0f + 0.75f * r);
+    return n <= 2.0f ? 2 : n <= four ? 4 : 32;
 }
 
 namespace {
@@ -528,7 +541,8 @@ void launch_propagate(const PropParams& P, int fused, cudaStream_t st)
         else launch_pass_counted<false>(Q, st);
     } else {
         Q.dual = 1;
-        Q.owners = prop_owners(P.V.W, P.V.H);
+        const long long own = (long long)P.V.W * P.V.H;
+        Q.owners = prop_owners(P.load > own ? P.load : own, P.V.r, PMH, P.load > own);
         if (Q.owners <= WARP_KLT) Q.list = nullptr;
         if (fused) launch_pass<true>(Q, st);
         else launch_pass<false>(Q, st);

@@ -474,7 +474,7 @@ void launch_iter(float4* out, const float4* in, float4* steps, const Views& V, f
         k_iter<true><<<tile_grid(V.W, V.H), dim3(BX, BY), 0, st>>>(out, in, V, dmax, iter, counts);
         return;
     }
-    const int owners = prop_owners(V.W, V.H);
+    const int owners = prop_owners((long long)V.W * V.H, V.r, VPM, false);
     const dim3 b(32, PT / 32), g((V.W + owners - 1) / owners, (V.H + PT / 32 - 1) / (PT / 32));
     if (owners > WARP_KLT) {
         const int blocks = (int)(((size_t)V.W * V.H + PT - 1) / PT);

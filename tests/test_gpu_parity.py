@@ -292,7 +292,7 @@ def test_pair_plane_loops_match_oracle(D, orc, W, H, r, fused):
 
 @pytest.mark.parametrize("fused", [0, 1])
 @pytest.mark.parametrize("W,H,r", [(1, 1, 1), (37, 5, 32), (74, 80, 2), (75, 80, 5), (148, 80, 3), (149, 80, 4), (33, 400, 1),
-                                   (5, 9, 4), (6, 5, 4)])
+                                   (5, 9, 4), (6, 5, 4), (110, 74, 1), (111, 74, 1)])
 def test_propagate_over_pair_planes_matches_oracle(D, orc, W, H, r, fused):
     """One propagate pass from the planes of pair_planes: two, four and 32 pixels per warp (the bounds of
     prop_owners among the sizes), windows of several passes over the shared memory, shared and single rows
