@@ -215,3 +215,30 @@ def test_vpm_cpp_drop_in_matches_oracle(native, torch_cuda, orc, tmp_path):
     d = np.fromfile(str(outv), np.float32).reshape(64, 96)
     L, R = scene.generate(7, 96, 64, 6, 2.0, 20.0)
     assert bits_equal(d, orc.vpm_disparity_simple(L, R, 3, 4, 24.0)[0]).all()
+
+
+def test_vpm_one_pixel_windows_take_one_launch_a_pass(torch_cuda, native):
+    """r = 0: a pass is one kernel (five launches otherwise), counted as the nodes of captured calls of 4 and 5
+    iterations"""
+    from cuda.bindings import runtime as rt
+
+    from cvt_b200 import scene
+    from cvt_b200.vpm import VPMStereoCL
+
+    a, b = (dev(torch_cuda, i) for i in scene.generate(3, 120, 110, 4, 1.0, 10.0))
+
+    def nodes(r, iters):
+        v = VPMStereoCL(r, iters, 16.0)
+        want = v.disparity_simple(a, b)
+        torch_cuda.cuda.synchronize()
+        g = torch_cuda.cuda.CUDAGraph(keep_graph=True)
+        with torch_cuda.cuda.graph(g):
+            got = v.disparity_simple(a, b)
+        g.replay()
+        assert bits_equal(host(got), host(want)).all()
+        err, _, n = rt.cudaGraphGetNodes(rt.cudaGraph_t(g.raw_cuda_graph()), 0)
+        assert err == rt.cudaError_t.cudaSuccess
+        return n
+
+    assert nodes(0, 5) - nodes(0, 4) == 1
+    assert nodes(1, 5) - nodes(1, 4) > 1
