@@ -279,16 +279,16 @@ __global__ void k_colour(const uint8_t* __restrict__ img, size_t stride, int W, 
     out[(size_t)y * W + x] = f4(unorm8(p.x), unorm8(p.y), unorm8(p.z), unorm8(p.w));
 }
 
-// the window's weight sum, in the first frame's w component (the other components are only read)
-__global__ void k_weight_sum(float4* c1, int W, int H, int r)
+// the first frame's plane: its colours, and in w the window's weight sum
+__global__ void k_weight_sum(float4* __restrict__ c1, const float4* __restrict__ colour, int W, int H, int r)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= W) return;
-    const float4 vc = c1[(size_t)y * W + x];
+    const float4 vc = colour[(size_t)y * W + x];
     float sum = 0.0f;
     for (int iy = max(y - r, 0); iy <= min(y + r, H - 1); iy++)
-        for (int ix = max(x - r, 0); ix <= min(x + r, W - 1); ix++) sum += weight(vc, c1[(size_t)iy * W + ix]);
-    reinterpret_cast<float*>(c1 + (size_t)y * W + x)[3] = sum;
+        for (int ix = max(x - r, 0); ix <= min(x + r, W - 1); ix++) sum += weight(vc, colour[(size_t)iy * W + ix]);
+    c1[(size_t)y * W + x] = f4(vc.x, vc.y, vc.z, sum);
 }
 
 // the quad plane of the second frame (Frames)
@@ -474,8 +474,8 @@ size_t quad_bytes(int W, int H) { return (size_t)(W + 1) * (H + 1) * sizeof(uint
 void launch_frames(float4* c1, float4* c2, uint4* quad, const uint8_t* img0, const uint8_t* img1, int W, int H, size_t stride,
                    int r, cudaStream_t st)
 {
-    launch_colour(img0, stride, W, H, c1, st);
-    k_weight_sum<<<row_grid(W, H), 128, 0, st>>>(c1, W, H, r);
+    launch_colour(img0, stride, W, H, c2, st);   // the first frame's colours, in c2 until they are read
+    k_weight_sum<<<row_grid(W, H), 128, 0, st>>>(c1, c2, W, H, r);
     launch_colour(img1, stride, W, H, c2, st);
     k_quad<<<row_grid(W + 1, H + 1), 128, 0, st>>>(img1, stride, W, H, quad);
 }
