@@ -446,3 +446,15 @@ def test_autotuner_keeps_the_fastest_candidate():
         assert all(c[1:] == (1, 1) for c in pm.calls)
     assert len({label(c) for c in DEFAULT_CANDIDATES}) == len(DEFAULT_CANDIDATES)
 
+    # by default the probe runs long enough to see what branched leaves out from the second iteration on (3 and 9:
+    # times of six uneven pairs on B200; 1: a lead within what two runs differ by)
+    pm = FakeHandle()
+
+    def by_iteration(fn):
+        fn()
+        branched = {1: 87.4, 3: 234.0, 9: 608.0}, {1: 87.2, 3: 255.0, 9: 723.0}
+        return branched[0 if pm.state[0] == "branched" else 1][pm.calls[-1][1]]
+
+    res = tune_batch(pm, [], [], [], [], timer=by_iteration)
+    assert res["best"]["schedule"] == "branched" and pm.state[0] == "branched"
+
