@@ -657,10 +657,11 @@ def test_primal_dual_steps_ragged_sizes(D, orc, W, H):
         assert bits_equal(host(o), orc.huber(inp, dt, lam, 1e-4, iters)).all(), ("huber", iters)
 
 
-@pytest.mark.parametrize("W,H", [(577, 256), (593, 257)])
+@pytest.mark.parametrize("W,H", [(577, 256), (593, 257), (1184, 128), (1183, 127), (1056, 144), (1055, 143)])
 def test_primal_dual_steps_both_tiles(D, orc, W, H):
-    """The largest image of the small smoothing tile (296 tiles of 32x16 or fewer: 19 x 16 = 304 is past it, as
-    is 19 x 17) and ragged edges of the large one, on finite fields"""
+    """Both smoothing tiles on finite fields: 304 and 323 tiles of 32x16, 296 (the largest image of the small tile)
+    and 297 (the smallest of the large one), the last two with ragged edges as well; each size and one a tile
+    smaller in both directions"""
     for w, h in ((W, H), (W - 32, H - 16)):
         rng = np.random.default_rng(w * 131 + h)
         inp = rng.standard_normal((h, w, 4)).astype(np.float32)
