@@ -1,5 +1,5 @@
-// Device functions of the PatchMatch-Huber path: plane-state algebra, support
-// weights and the bilinear row read.  Each function names the reference lines it computes
+// Device functions of the PatchMatch-Huber path: plane-state algebra and support
+// weights.  Each function names the reference lines it computes
 // (cvt/cl/kernel/pmhstereo.cl, Matrix3.cl).  Arithmetic is FP32 with the
 // reference's operation order; the file must be compiled with -fmad=false so
 // that only the explicit fmaf() calls (the "hot" sites, enabled by the template
@@ -159,12 +159,6 @@ __device__ __forceinline__ float2 smooth_distance(float4 sa, float4 sb, float4 s
     return make_float2(smooth_dist1(sa, smooth, cx, cy, dmax, lr), smooth_dist1(sb, smooth, cx, cy, dmax, lr));
 }
 
-__device__ __forceinline__ uint32_t signbits4(float4 v)
-{
-    return (__float_as_uint(v.x) >> 31) | ((__float_as_uint(v.y) >> 31) << 1) | ((__float_as_uint(v.z) >> 31) << 2) |
-           ((__float_as_uint(v.w) >> 31) << 3);
-}
-
 // grey weights of pmhstereo.cl:670
 #define PM_GW_R 0.2126f
 #define PM_GW_G 0.7152f
@@ -215,24 +209,6 @@ template <bool F>
 __device__ __forceinline__ float support_weight_any(float dx, float dy, float dz)
 {
     return expf_(-fabsf(gray_dot<F>(dx, dy, dz)) * 12.0f);
-}
-
-// SAMPLER_BILINEAR (:71) read at (u, row + 0.5): OpenCL 1.2 s8.2 with the vertical
-// weight exactly 0, i.e. (1-a)*T[i0] + a*T[i0+1], columns clamped to the edge
-template <bool F>
-__device__ __forceinline__ float4 lerp_row(const float4* __restrict__ row, int W, float u)
-{
-    const float t = u - 0.5f;
-    if (!fin(t)) { const float n = qnan(); return f4(n, n, n, n); }
-    float fl = floorf(t);
-    const float a = t - fl;
-    fl = fminf(fmaxf(fl, -1.0f), (float)W);
-    const int i0 = (int)fl;
-    const int j0 = min(max(i0, 0), W - 1), j1 = min(max(i0 + 1, 0), W - 1);
-    const float4 T0 = __ldg(row + j0), T1 = __ldg(row + j1);
-    const float b = 1.0f - a;
-    if (F) return f4(fmaf(a, T1.x, b * T0.x), fmaf(a, T1.y, b * T0.y), fmaf(a, T1.z, b * T0.z), fmaf(a, T1.w, b * T0.w));
-    return f4(b * T0.x + a * T1.x, b * T0.y + a * T1.y, b * T0.z + a * T1.z, b * T0.w + a * T1.w);
 }
 
 }  // namespace pm

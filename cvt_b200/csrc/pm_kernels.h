@@ -72,7 +72,7 @@ void prop_tile_shape(int* w, int* h);
 // false for any other width
 bool prop_batch_tile_shape(int tile_w, int* w, int* h);
 // pairs per batched propagate launch: their arguments are one kernel parameter block
-// (128 x 208 bytes, within the 32,764 bytes a launch may pass)
+// (128 x 224 bytes, within the 32,764 bytes a launch may pass)
 constexpr int PROP_GROUP = 128;
 struct PropGroup {
     PropParams p[PROP_GROUP];

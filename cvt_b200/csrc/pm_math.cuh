@@ -165,18 +165,6 @@ PM_HD float acospif_(float x)
     return a * 0.318309873342514038f;
 }
 
-// x / 0.05f correctly rounded for 0 <= x <= 0.05: one multiply by RN(1/0.05) = 20 and
-// one fma correction (Markstein); verified against IEEE division for every float in
-// [2^-103, 0.05] and 0; smaller inputs take the division.
-PM_HD float div005(float x)
-{
-    const float q = x * 20.0f;
-    const float r = fmaf(-q, 0.05f, x);
-    float res = fmaf(r, 20.0f, q);
-    if (x < 7.88860905e-31f) res = x / 0.05f;   // 2^-100
-    return res;
-}
-
 // Smallest float c >= 0 with RN(c / b) >= m, for finite b >= 1: the cost loop's test
 // `census / bilw >= mincost` (pmhstereo.cl:724) is equivalent to census >= threshold
 // because c -> RN(c / b) is monotone.  m <= 0 gives -inf (always), NaN m gives NaN

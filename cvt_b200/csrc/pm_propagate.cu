@@ -27,7 +27,7 @@ namespace {
 #endif
 constexpr int PROP_BX = 32, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
 // Resident threads per SM asked of the register allocator for each kernel (640 = 96 registers, no
-// spills).  The window loops issue 88-92% of the cycles, so more threads give nothing: 1280x720,
+// spills).  The window loops issue 81-88% of the cycles (640x360), so more threads give nothing: 1280x720,
 // r = 10, 3 iterations, ms (chain / Gauss-Newton): 512 threads 75.5 / 89.1, 640 69.2 / 88.9,
 // 768 69.2 / 88.7, 1024 (chain) 71.5; unrolling a row's loop by two 75.0 / 89.2 at 512.  The
 // block shape does not matter either (32x4, 16x8, 8x16 and 32x2 within 1.5% of each other).
@@ -445,7 +445,7 @@ void launch_propagate_batch(const PropParams* group, int n, const JobList& J, in
                             int counting, int* next, cudaStream_t st)
 {
     if (J.njobs <= 0 || n < 1 || n > PROP_GROUP) return;
-    static thread_local PropGroup tab;   // 23 KB: off the stack; copied into the launch
+    static thread_local PropGroup tab;   // 28 KB: off the stack; copied into the launch
     for (int i = 0; i < n; i++) {
         tab.p[i] = group[i];
         tab.p[i].owners = tile_w;

@@ -15,14 +15,14 @@
 //
 // A pass is three kernels, as the main path's (candidates, Gauss-Newton steps, their evaluation), over the
 // pair-plane loops of pm_window.cuh / pm_warp.cuh.  The general loops below, one kernel per pass, count the
-// taps (pm_vpm_set_counting) and serve injected gradients that are not finite.  Measured at 640x480, r = 10,
+// taps (pm_vpm_set_counting) and serve windows of one pixel and injected gradients that are not finite.  Measured at 640x480, r = 10,
 // 8 iterations: general loops 95.7 ms a call, the three kernels 50.1 (30.1 + 15.9 + 3.1; 56.7 with the
 // Gauss-Newton steps of every pixel in every pass).
 //
 // Arithmetic is the reference's FP32 sequence (the file is compiled with -fmad=false): every
 // result equals the restatement in oracle/pm_oracle.cpp bit for bit.  The one double in the
-// source, the 0.25 literal of patch_census_klt (VPMStereo.cl:162), is kept: the tap cost is a
-// double sum rounded once to float.
+// source, the 0.25 literal of patch_census_klt (VPMStereo.cl:162), makes the tap cost a double sum rounded
+// once to float: the general loops form it so, the pair-plane loops as one fma that rounds the same (tap_cost).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -39,8 +39,8 @@ namespace vpm {
 
 constexpr float ALPHA = 0.05f;       // VPMStereo.cl:130, :210
 constexpr float WEIGHT = 8.0f;       // CENSUS_COLOR_WEIGHT (:30)
-// iterate / init blocks: a warp spans 32 columns of one row; k_iter asks for 3 resident blocks
-// per SM (80 registers): 13% faster than the compiler's 100-register choice at 2 blocks
+// blocks of the general loops (k_init, k_iter): a warp spans 32 columns of one row; k_iter asks for 3 resident
+// blocks per SM (80 registers): 13% faster than the compiler's 100-register choice at 2 blocks
 constexpr int BX = 32, BY = 8;
 
 typedef ViewData Views;
@@ -65,7 +65,7 @@ __device__ __forceinline__ float weight(float4 t, float4 ctr)
 }
 
 // (1 - a) T0 + a T1 per component, each product and the sum rounded once (SAMPLER_BILINEAR
-// with the vertical weight 0, as lerp_row)
+// with the vertical weight 0)
 __device__ __forceinline__ float4 mix4(float a, float4 T0, float4 T1)
 {
     const float b = 1.0f - a;
@@ -73,7 +73,7 @@ __device__ __forceinline__ float4 mix4(float a, float4 T0, float4 T1)
               __fadd_rn(__fmul_rn(b, T0.z), __fmul_rn(a, T1.z)), __fadd_rn(__fmul_rn(b, T0.w), __fmul_rn(a, T1.w)));
 }
 
-// colour and gradient of the second image at (u, row + 0.5): lerp_row of both planes
+// colour and gradient of the second image at (u, row + 0.5): both planes interpolated
 __device__ __forceinline__ void sample2(const Views& V, int row, float u, float4& c, float4& g)
 {
     const float t = u - 0.5f;

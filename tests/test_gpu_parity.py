@@ -1,8 +1,7 @@
 """Parity of the sm_100a kernels with the oracle, through the C ABI.
 
-strict mode (fused=0) must reproduce the reference-kernel golden fixtures bit
-for bit; fused mode (the default) must reproduce the oracle's fused
-restatement bit for bit.  NaN payloads are not compared (every NaN equals
+strict mode (fused=0, the default) must reproduce the reference-kernel golden fixtures
+bit for bit; fused mode must reproduce the oracle's fused restatement bit for bit.  NaN payloads are not compared (every NaN equals
 every NaN).  Larger sizes are checked against the oracle where it finishes in
 seconds and through size-independent properties beyond that.
 """
@@ -740,7 +739,7 @@ def test_hd_strict_matches_reference_fixture(native, torch_cuda):
 def test_small_config_strict_exact_fused_within_tolerance(native, torch_cuda, orc):
     """The 320x240 / 15x15 / 4 (5) iterations / left-view workload at full size.  Strict GPU equals
     the strict restatement (= the reference kernels) bit for bit.  Fused GPU against the same:
-    north_star's tolerance (planes equal except FP32 ties, disparity within 1e-3 px, cost within
+    the workload's tolerance (planes equal except FP32 ties, disparity within 1e-3 px, cost within
     1e-4 relative) holds only where the fma-contracted trajectory has not diverged; the test pins
     the measured share (about 86%) from below and records it."""
     from cvt_b200 import PMHuberStereo, scene
