@@ -526,7 +526,7 @@ def run_vpm(args, wl, rank, world, local):
     if os.path.exists(tfile):
         traffic = json.load(open(tfile)).get("bytes_per_launch")
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-            "frac": (achieved / peak) if peak else None, "traffic": traffic, "kernel": "k_iter (vpmstereo_iter_simple)",
+            "frac": (achieved / peak) if peak else None, "traffic": traffic, "kernel": "k_cand + k_steps_list + k_settle_list (vpmstereo_iter_simple)",
             "avg_launch_ms": iter_ms, "flops_per_launch": flops_launch,
             "peak_source": "FP32 fma probe measured in this run (pm_measure_fp32_peak)"}
     line = {"metric": METRIC, "value": value, "unit": "Mpixel·iterations/s", "n_gpus": world, "steps": args.steps,
@@ -537,7 +537,7 @@ def run_vpm(args, wl, rank, world, local):
                        "l2": "flushed between steps (256 MiB write)"},
             "e2e": {"value": e2e_value, "unit": "Mpixel·iterations/s", "h2d_bytes_per_step": 2 * W * H * 4,
                     "d2h_bytes_per_step": W * H * 4},
-            "roofline": roof, "clocks": clk, "gpu_launches": (4 + iters) * args.steps,
+            "roofline": roof, "clocks": clk, "gpu_launches": (6 + 4 * iters) * args.steps,
             "counters": {"cost_taps": taps[0], "gn_taps": taps[1]},
             "phase_ms": {"iterations": iter_ms * iters, "rest": statistics.median(base_ms)}}
     if rank == 0 and world == 1 and not args.no_cpu:
@@ -640,7 +640,7 @@ def run_svpm(args, wl, rank, world, local):
                        "l2": "flushed between steps (256 MiB write)"},
             "e2e": {"value": e2e_value, "unit": metric, "h2d_bytes_per_step": 2 * W * H * 4,
                     "d2h_bytes_per_step": W * H * 8},
-            "roofline": roof, "clocks": clk, "gpu_launches": (4 + passes) * args.steps,
+            "roofline": roof, "clocks": clk, "gpu_launches": (6 + passes) * args.steps,
             "counters": {"cost_taps": taps},
             "phase_ms": {"passes": pass_ms * passes, "rest": statistics.median(base_ms)}}
     if rank == 0 and world == 1 and not args.no_cpu:
@@ -909,7 +909,7 @@ def measure_disparity(args, wl, pm, call, dL, dR, L, R, local, world, levels, ru
     achieved = flops_launch / avg_launch_s / 1e12
     roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": (achieved / peak) if peak else None, "traffic": None,
-            "kernel": "propagate pass (k_prop_chain + k_prop_klt + k_prop_final)", "avg_launch_ms": avg_launch_s * 1e3,
+            "kernel": "propagate pass (k_prop_chain + k_prop_klt_list + k_prop_final)", "avg_launch_ms": avg_launch_s * 1e3,
             "flops_per_launch": flops_launch,
             "peak_source": "FP32 fma probe measured in this run (pm_measure_fp32_peak)"}
     return {"value": value, "ms_per_step": total_ms / steps, "e2e_value": e2e_value, "roofline": roof, "clocks": clk,
