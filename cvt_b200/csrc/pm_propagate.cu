@@ -27,7 +27,7 @@ namespace {
 #endif
 constexpr int PROP_BX = 32, PROP_BY = PM_PROP_BY, PROP_THREADS = PROP_BX * PROP_BY;
 // Resident threads per SM asked of the register allocator for each kernel (640 = 96 registers, no
-// spills).  The window loops issue 81-88% of the cycles (640x360), so more threads give nothing: 1280x720,
+// spills).  The window loops issue 82-88% of the cycles (640x360), so more threads give nothing: 1280x720,
 // r = 10, 3 iterations, ms (chain / Gauss-Newton): 512 threads 75.5 / 89.1, 640 69.2 / 88.9,
 // 768 69.2 / 88.7, 1024 (chain) 71.5; unrolling a row's loop by two 75.0 / 89.2 at 512.  The
 // block shape does not matter either (32x4, 16x8, 8x16 and 32x2 within 1.5% of each other).
