@@ -34,9 +34,9 @@ PatchMatch and its disparity within 1 px of it on >= 98% of the pixels plain
 PatchMatch keeps (LR check); value = that time in ms (null if no k up to 9 reaches it).
 
 `--impl reference` times the reference's CPU implementation instead: the
-reference kernel sources compiled through the OpenCL-C shim (oracle/_ref) when
-built, otherwise the CPU restatement (oracle/), on a bounded crop of the same
-workload, using every host thread.
+reference kernel sources compiled through the OpenCL-C shim (oracle/_ref), on a
+bounded crop of the same workload, using every host thread; where they are not
+built (no reference source tree) it prints an "unavailable" line.
 """
 import argparse
 import json
@@ -202,7 +202,12 @@ def run_reference(args, wl, rank, world):
     if rank != 0:
         return
     from cvt_b200 import scene
+    from oracle.pyoracle import available
 
+    if not available("ref"):   # never this project's own restatement in its place
+        print(json.dumps({"impl": "reference", "unavailable": "the reference kernels are not compiled on this host "
+                                                              "(no reference source tree)"}))
+        return
     W, H, npl, dlo, dhi, r, dmax, iters, views, pp = wl
     crop = REF_CROP[args.config]
     L, R = scene.generate(0, crop[0], crop[1], max(2, npl * crop[0] * crop[1] // (W * H) + 2), dlo, dhi)
